@@ -316,42 +316,6 @@ ozgb_status choose_config(ozgb_handle h, const Operands &o, int mode, cudaStream
     return OZGB_OK;
 }
 
-// GEMM launch arguments that follow from the plan alone (shared by all problems
-// of a grouped launch); operands, sizes and tiles are set by the caller.
-void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, unsigned long long timeout_ns) {
-    memset(g, 0, sizeof *g);
-    g->KC = p.KC;
-    g->s = p.cfg.s;
-    g->J = p.cfg.J;
-    g->b = p.cfg.b;
-    g->out_mode = out_mode;
-    g->stages = p.stages;
-    g->stage_bytes = p.stage_bytes;
-    g->a_block_bytes = p.a_block_bytes;
-    g->b_block_bytes = p.b_block_bytes;
-    g->b_pad_lo_bytes = static_cast<uint32_t>(p.pad_lo) * p.b_slice_bytes;
-    g->b_region_bytes = p.b_region_bytes;
-    g->tmem_cols = p.tmem_cols;
-    g->err = err;
-    g->timeout_ns = timeout_ns;
-    g->alpha = 1.0;
-    g->beta = 0.0;
-    g->n_acc = p.n_acc;
-    g->n_iss = p.n_iss;
-    for (int a = 0; a < kMaxAcc; ++a) g->acc_t0[a] = p.acc_t0[a];
-    g->G = p.G;
-    for (int i = 0; i < p.G; ++i) {
-        g->blk_lo[i] = p.blk_lo[i];
-        g->blk_nb[i] = p.blk_nb[i];
-        g->blk_p0[i] = p.blk_p0[i];
-        g->blk_p1[i] = p.blk_p1[i];
-        g->blk_period[i] = p.blk_period[i];
-        g->blk_off[i] = p.blk_off[i];
-        g->blk_col1[i] = p.blk_col1[i];
-    }
-    g->dbl_mask = p.dbl_mask;
-}
-
 // Auxiliary streams and their events, created on first use.
 ozgb_status ensure_aux(ozgb_handle h) {
     if (h->ev_fork) return OZGB_OK;
@@ -695,7 +659,7 @@ struct GroupLaunch {
 
 // The launch-level fields of a plan's GemmArgs as a fixed array (no allocation):
 // problems with equal arrays share a grouped launch.
-constexpr int kLaunchFields = 18 + kMaxAcc + 7 * kMaxGroups;
+constexpr int kLaunchFields = 16 + kMaxAcc + 5 * kMaxGroups;
 struct LaunchFields {
     long long v[kLaunchFields];
     int n = 0;
@@ -703,14 +667,13 @@ struct LaunchFields {
 };
 LaunchFields launch_fields(const GemmArgs &g, const Plan &p) {
     LaunchFields f;
-    const long long head[18] = {reinterpret_cast<long long>(p.fn), static_cast<long long>(p.smem), g.KC, g.s, g.J,
+    const long long head[16] = {reinterpret_cast<long long>(p.fn), static_cast<long long>(p.smem), g.KC, g.s, g.J,
                                 g.b, g.out_mode, g.stages, g.stage_bytes, g.a_block_bytes, g.b_block_bytes,
-                                g.b_pad_lo_bytes, g.b_region_bytes, g.tmem_cols, g.n_acc, g.n_iss, g.G, g.dbl_mask};
+                                g.tmem_cols, g.n_acc, g.n_iss, g.G, g.dbl_mask};
     for (long long x : head) f.v[f.n++] = x;
     for (int a = 0; a < kMaxAcc; ++a) f.v[f.n++] = g.acc_t0[a];
     for (int i = 0; i < g.G; ++i)
-        for (long long x : {g.blk_lo[i], g.blk_nb[i], g.blk_p0[i], g.blk_p1[i], g.blk_period[i], g.blk_off[i],
-                            g.blk_col1[i]})
+        for (long long x : {g.blk_lo[i], g.blk_nb[i], g.blk_period[i], g.blk_off[i], g.blk_col1[i]})
             f.v[f.n++] = x;
     unsigned long long h = 1469598103934665603ull;  // FNV-1a over the words
     for (int i = 0; i < f.n; ++i) h = (h ^ static_cast<unsigned long long>(f.v[i])) * 1099511628211ull;

@@ -8,8 +8,8 @@
 //   int128 -> double reconstruction                include/oz_aie.h:92-150
 //
 // GB300 design (persistent CTAs, one per SM, each looping over 128 x BN tiles of
-// C; 640 threads: a producer warp, 16 drain/epilogue warps and up to three
-// MMA-issuing warps on three schedulers):
+// C; 640 threads: a producer warp, up to three MMA-issuing warps on three schedulers
+// and 16 drain/epilogue warps):
 //   * Carrier: tcgen05.mma kind::f16 with bf16 slices (|v| <= 127 is exact in
 //     bf16) and fp32 accumulators in TMEM.  (kind::i8 is not accepted by ptxas
 //     for sm_103a.)  Slices of b <= 4 bits may instead be e4m3 (kind::f8f6f4,
@@ -20,36 +20,35 @@
 //     pairs_in_bin(j) * KB_j * (2^b-1)^2 <= 2^24, so the fp32 accumulation is exact.
 //   * TMEM holds one fp32 accumulator of BN columns per bin j (column j*BN), and
 //     a second range for each double-buffered block where the columns allow it.
-//     Bins are partitioned into up to 8 blocks of at most 256 columns.  Every
-//     UMMA of a block spans the whole block: A slice p against the B slices
-//     q = j - p of all bins j of the block, which are consecutive in shared
-//     memory; q outside [0, s) reads zero slices padded below and above the
-//     loaded ones.  On GB300 one M=128, K=16 UMMA occupies the tensor pipe for
-//     N/2 cycles, and one issuing thread issues one about every 80-100 cycles,
-//     so wide UMMAs from several issuers feed the pipe; the planner picks the
-//     partition with a cost model fitted to this kernel.
-//   * The UMMA runs of a K step (block, A slice) are dealt round-robin to the
-//     issuing warps, which all accumulate (enable_input_d = 1): the drain warps
-//     store zeros over every accumulator they read out, and TMEM starts zeroed.
-//   * Each block is a drain group with its own period (its tightest bin).  In
-//     each chunk the issuers first issue the blocks that drain after this chunk,
-//     then the others, and last the blocks drained after the previous chunk
-//     (after waiting for their drain): a drain overlaps the UMMAs of the other
-//     blocks.  A double-buffered block switches ranges at each drain instead.
-//   * Drain (warps 2..17): TMEM -> registers, fp32 -> int32 (exact), then one
+//     Bins are partitioned into up to 8 blocks of at most 256 columns.  A UMMA
+//     takes A slice p against the B slices q = j - p of the bins j of one block,
+//     which are consecutive in shared memory, and covers exactly the bins that
+//     hold a pair.  On GB300 a M=128, K=16 UMMA of N columns takes
+//     max(N/2, 32 + N/4) cycles (the tensor pipe, or its operands from shared
+//     memory at 128 bytes a cycle).
+//   * Each block belongs to one issuing warp, so its UMMAs run in order and the
+//     first one after a drain overwrites the accumulator.  Issuers do not wait for
+//     one another beyond the stage ring.
+//   * Each block is a drain group with its own period (its tightest bin).  A block
+//     whose accumulator is being read out holds up its own issuer only; a
+//     double-buffered block switches ranges at each drain instead.
+//   * Drain (warps 4..19): TMEM -> registers, fp32 -> int32 (exact), then one
 //     32 x 32 -> 64-bit multiply-add by 2^rel into the 64-bit accumulator of the
 //     bin's group (consecutive bins whose weights relative to the group's first
-//     bin stay <= 2^30).  The W-word exact sum is assembled once per element in
-//     the epilogue.  Integer ALU work competes with the MMA-issuing warps on their
-//     schedulers, so the drain keeps it to two instructions per value.
+//     bin stay <= 2^30).  The buffer is released as soon as its last bin is in
+//     registers.
 //   * The last partial wave of a launch may be split along K (split_parts): the
 //     parts add their 64-bit group sums into global scratch with atomics and
 //     the part that completes a tile's count rounds and stores it.
-//   * Epilogue: the exact accumulator q is rounded once to FP64 with the scale
+//   * Epilogue: the exact sum is rounded once to FP64 with the scale
 //     2^{Er+Ec-2044-b(J+1)} (round-to-nearest, or the reference's truncating
 //     decode, or written raw for parity dumps).
 //   * Every mbarrier wait is bounded (globaltimer); on expiry the kernel records
 //     an error code, waits for its own copies and MMAs, frees TMEM and returns.
+//
+// At 4096^3 (s = 8, p + q <= 8, 2752 tiles of 128 x 48) the launch takes 3.7 ms:
+// 1600 cycles per K step of a tile, of which the UMMAs need 1104.  Without drains it
+// takes 1280; the rest is the issuers and drain warps sharing the schedulers.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -69,28 +68,20 @@ __device__ __forceinline__ long long mad_wide(int32_t a, int32_t m, long long c)
 }
 
 // acc[i][A] += v[i] * 2^rel modulo 2^64 for NV fp32 values holding exact
-// integers (|v| <= 2^24).  Exact-mode plans keep rel <= 30; the paired output
-// of the reference (sums modulo 2^64) may need up to 63.
+// integers (|v| <= 2^24).  Exact-mode plans keep rel <= 30; the paired output of the
+// reference (sums modulo 2^64) may need up to 63.  (An FP32 add of 1.5 2^23 instead of
+// F2I, for values below 2^22, measured 1 % slower: the check costs what it saves.)
 template <int NA, int A, int NV>
 __device__ __forceinline__ void acc_add(long long (*acc)[NA], const uint32_t *v, int rel) {
     if (rel <= 30) {
         const int32_t m = 1 << rel;
 #pragma unroll
         for (int i = 0; i < NV; ++i) acc[i][A] = mad_wide(__float2int_rz(__uint_as_float(v[i])), m, acc[i][A]);
-    } else if (rel <= 36) {
-        const int k = rel - 30;  // |v| 2^k < 2^31
+    } else {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const uint32_t iv = static_cast<uint32_t>(__float2int_rz(__uint_as_float(v[i])));
-            acc[i][A] = mad_wide(static_cast<int32_t>(iv << k), 1 << 30, acc[i][A]);
-        }
-    } else if (rel < 64) {
-        const int k = rel - 32;  // only the high word changes (modulo 2^64)
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const uint32_t iv = static_cast<uint32_t>(__float2int_rz(__uint_as_float(v[i])));
-            acc[i][A] += static_cast<long long>(static_cast<unsigned long long>(iv << k) << 32);
-        }
+        for (int i = 0; i < NV; ++i)
+            acc[i][A] += static_cast<long long>(
+                static_cast<unsigned long long>(static_cast<long long>(__float2int_rz(__uint_as_float(v[i])))) << rel);
     }
 }
 
@@ -107,182 +98,133 @@ __device__ __forceinline__ void acc_add_group(long long (*acc)[NA], const uint32
     }
 }
 
-// q += x * 2^sh for a signed 64-bit x, q two's complement in W words (epilogue).
-template <int W>
-__device__ __forceinline__ void q_add_i64(uint32_t (&q)[W], long long x, int sh) {
-    const int k = sh >> 5, r = sh & 31;
-    const uint32_t lo = static_cast<uint32_t>(x);
-    const uint32_t hi = static_cast<uint32_t>(static_cast<unsigned long long>(x) >> 32);
-    const uint32_t ext = static_cast<uint32_t>(x >> 63);
-    const uint32_t p0 = lo << r, p1 = __funnelshift_l(lo, hi, r), p2 = __funnelshift_l(hi, ext, r);
-    uint32_t carry = 0;
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-        const int d = w - k;
-        const uint32_t a = d < 0 ? 0u : d == 0 ? p0 : d == 1 ? p1 : d == 2 ? p2 : ext;
-        const unsigned long long sum = static_cast<unsigned long long>(q[w]) + a + carry;
-        q[w] = static_cast<uint32_t>(sum);
-        carry = static_cast<uint32_t>(sum >> 32);
-    }
-}
-
-// TMEM columns per load batch of a drain thread: the widest that divides its
-// columns and leaves the accumulators (2 NA registers per column) room.
-__host__ __device__ constexpr int drain_batch(int cols, int acc_regs) {
-    return (cols % 16 == 0 && acc_regs + 16 <= 64)   ? 16
-           : (cols % 12 == 0 && acc_regs + 12 <= 64) ? 12
-           : (cols % 8 == 0 && acc_regs + 8 <= 64)   ? 8
-                                                     : 4;
-}
-
 // ------------------------------------------------------------ q -> double
-template <int W>
-__device__ __forceinline__ uint32_t qword(const uint32_t (&m)[W], int i) {
-    uint32_t r = 0;
+// The exact sum of an element's accumulator groups, sum_x acc[x] 2^B[x] (B[0] = 0),
+// as a 128-bit window and what lies below it: value = (S + f) 2^low with 0 <= f < 1
+// and sticky = (f != 0).  The bits of a group above the next group's weight are first
+// carried into that group (the groups are at most 37 bits apart and stay below 2^62);
+// then the window takes the groups from the top.  A group that no longer fits (|S| is
+// then past 2^64, well over the 53 bits of a result) only sets sticky.
+template <int NA>
+OZ_HD inline void acc_window(const long long (&acc)[NA], int n_acc, const int (&B)[kMaxAcc], __int128 *S_out,
+                             bool *sticky_out, int *low_out) {
+    long long top = acc[0];
+    unsigned long long dig[NA];  // dig[x]: group x's bits below group x + 1's weight
 #pragma unroll
-    for (int t = 0; t < W; ++t) r = (t == i) ? m[t] : r;
-    return r;
-}
-// floor(m / 2^sh) for sh >= 0 (low 64 bits), m << -sh for sh < 0.
-template <int W>
-__device__ __forceinline__ uint64_t qextract64(const uint32_t (&m)[W], int sh) {
-    if (sh < 0) {
-        const uint64_t lo = static_cast<uint64_t>(m[0]) | (W > 1 ? (static_cast<uint64_t>(m[1]) << 32) : 0ull);
-        return (-sh >= 64) ? 0ull : (lo << (-sh));
-    }
-    const int wi = sh >> 5, bo = sh & 31;
-    const uint32_t w0 = qword(m, wi), w1 = qword(m, wi + 1), w2 = qword(m, wi + 2);
-    const uint32_t lo = __funnelshift_r(w0, w1, bo);
-    const uint32_t hi = __funnelshift_r(w1, w2, bo);
-    return (static_cast<uint64_t>(hi) << 32) | lo;
-}
-template <int W>
-__device__ __forceinline__ int qbit(const uint32_t (&m)[W], int i) {
-    if (i < 0) return 0;
-    return static_cast<int>((qword(m, i >> 5) >> (i & 31)) & 1u);
-}
-template <int W>
-__device__ __forceinline__ bool qany_below(const uint32_t (&m)[W], int i) {
-    uint32_t acc = 0;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-        const int base = 32 * t;
-        if (base + 32 <= i) acc |= m[t];
-        else if (base < i) acc |= m[t] & ((1u << (i - base)) - 1u);
-    }
-    return acc != 0;
-}
-
-// value = q * 2^(escale - 2044 - bJ1), q two's complement in W words.
-template <int W>
-__device__ __forceinline__ double q_to_double(const uint32_t (&q)[W], int escale, int bJ1, int mode) {
-    const bool neg = static_cast<int32_t>(q[W - 1]) < 0;
-    uint32_t m[W];
-    {
-        uint32_t carry = 1;
-#pragma unroll
-        for (int t = 0; t < W; ++t) {
-            const uint32_t x = neg ? ~q[t] : q[t];
-            const uint32_t add = neg ? carry : 0u;
-            const uint32_t s = x + add;
-            carry = (neg && s < x) ? 1u : 0u;
-            m[t] = s;
+    for (int x = 1; x < NA; ++x)
+        if (x < n_acc) {
+            const int d = B[x] - B[x - 1];
+            dig[x - 1] = static_cast<unsigned long long>(top) & ((1ull << d) - 1ull);
+            top = acc[x] + (top >> d);
         }
-    }
-    int L = 0;
+    __int128 S = top;
+    bool sticky = false, full = false;
+    int low = B[n_acc - 1];
 #pragma unroll
-    for (int t = 0; t < W; ++t)
-        if (m[t]) L = 32 * t + 32 - __clz(m[t]);
-    if (L == 0) return 0.0;
-    uint64_t bits;
-    if (mode == OUT_RZ_REF) {
-        // include/oz_aie.h:129-146: exponent = L - b(d+1) - 1, truncate to 53 bits,
-        // lu = mant - 2^52 + sign + (exponent+1023)<<52 + (Er+Ec+2-2046)<<52 mod 2^64.
-        const long long exponent = static_cast<long long>(L) - bJ1 - 1;
-        uint64_t lu = qextract64(m, L - 53);
-        lu -= 0x0010000000000000ull;
-        lu += (neg ? 0x8000000000000000ull : 0ull) + (static_cast<uint64_t>(exponent + 1023) << 52) +
-              (static_cast<uint64_t>(static_cast<long long>(escale) - 2044) << 52);
-        bits = lu;
-    } else {
-        const int e2 = escale - 2044 - bJ1;
-        const int biased = L - 1 + e2 + 1023;
-        const int sh = (biased >= 1) ? L - 53 : L - 53 + (1 - biased);
-        uint64_t mm = (sh > L) ? 0ull : qextract64(m, sh);
-        const int rb = (sh - 1 >= L) ? 0 : qbit(m, sh - 1);
-        const bool st = qany_below(m, sh - 1);
-        if (rb && (st || (mm & 1ull))) mm++;
-        if (biased >= 1) {
-            if (biased >= 2047) {
-                bits = 0x7FF0000000000000ull;
+    for (int x = NA - 1; x >= 1; --x)
+        if (x < n_acc) {
+            const int d = B[x] - B[x - 1];
+            const long long hi = static_cast<long long>(S >> 64);
+            // the first of these fits: |top| < 2^63; else |S| < 2^(126 - d)
+            if (x == n_acc - 1 || (!full && ((hi ^ (hi >> 63)) >> (62 - d)) == 0)) {
+                S = static_cast<__int128>(static_cast<unsigned __int128>(S) << d) +
+                    static_cast<__int128>(dig[x - 1]);
+                low = B[x - 1];
             } else {
-                bits = (static_cast<uint64_t>(biased - 1) << 52) + mm;
-                if (bits >= 0x7FF0000000000000ull) bits = 0x7FF0000000000000ull;
+                full = true;
+                sticky = sticky || dig[x - 1] != 0;
             }
-        } else {
-            bits = mm;
         }
-        if (neg) bits |= 0x8000000000000000ull;
-    }
-    return __longlong_as_double(static_cast<long long>(bits));
+    *S_out = S;
+    *sticky_out = sticky;
+    *low_out = low;
 }
 
-// The same rounding (OUT_RN) for q = a0 + a1 2^B with 0 <= B <= 63, the exact sum
-// of at most two accumulator groups: one signed 128-bit integer, so the rounding
-// needs no word selects.  Bit for bit the result of q_to_double.
-__device__ __forceinline__ double acc2_to_double_rn(long long a0, long long a1, int B, int escale, int bJ1) {
-    const __int128 S = static_cast<__int128>(a0) + (static_cast<__int128>(a1) << B);
-    if (S == 0) return 0.0;
+OZ_HD inline int clz64(unsigned long long x) {
+#if defined(__CUDA_ARCH__)
+    return __clzll(static_cast<long long>(x));
+#else
+    return __builtin_clzll(x);
+#endif
+}
+
+// Bits of the double nearest to h 2^(biased - 1086) (h normalised, its lowest bit
+// sticky) when the biased exponent is outside [1, 2046]: subnormal, zero or infinite.
+OZ_HD inline unsigned long long round_out_of_range(unsigned long long h, int biased) {
+    if (biased >= 2047) return 0x7FF0000000000000ull;
+    const int sh = 12 - biased;  // >= 12
+    if (sh > 64) return 0ull;
+    if (sh == 64) return h > 0x8000000000000000ull ? 1ull : 0ull;
+    unsigned long long mm = h >> sh;
+    const bool rb = ((h >> (sh - 1)) & 1ull) != 0, st = (h & ((1ull << (sh - 1)) - 1ull)) != 0;
+    if (rb && (st || (mm & 1ull))) ++mm;
+    return mm;
+}
+
+// Bits of (S + f) 2^e2 as a double: rounded to nearest even (OUT_RN) or the
+// reference's truncating decode (OUT_RZ_REF, include/oz_aie.h:129-146: 53 truncated
+// bits and the exponent added modulo 2^64).
+OZ_HD inline unsigned long long window_bits(__int128 S, bool sticky, int e2, int mode) {
     const bool neg = S < 0;
-    const unsigned __int128 m = neg ? static_cast<unsigned __int128>(-S) : static_cast<unsigned __int128>(S);
-    const unsigned long long hi = static_cast<unsigned long long>(m >> 64), lo = static_cast<unsigned long long>(m);
-    const int L = hi ? 128 - __clzll(static_cast<long long>(hi)) : 64 - __clzll(static_cast<long long>(lo));
-    const int e2 = escale - 2044 - bJ1;
-    const int biased = L - 1 + e2 + 1023;
-    const int sh = (biased >= 1) ? L - 53 : L - 53 + (1 - biased);
-    unsigned long long mm;
-    if (sh < 0) mm = (-sh >= 64) ? 0ull : (lo << (-sh));  // L < 53: m is lo
-    else mm = (sh > L) ? 0ull : static_cast<unsigned long long>(m >> sh);
-    const int rpos = sh - 1;  // the rounding bit's position
-    const int rb = (rpos < 0 || rpos >= L) ? 0 : static_cast<int>((m >> rpos) & 1u);
-    bool st = false;          // any bit below the rounding bit
-    if (rpos >= 128) st = true;  // m != 0
-    else if (rpos > 0) st = (m & ((static_cast<unsigned __int128>(1) << rpos) - 1u)) != 0;
-    if (rb && (st || (mm & 1ull))) mm++;
-    uint64_t bits;
-    if (biased >= 1) {
-        if (biased >= 2047) {
-            bits = 0x7FF0000000000000ull;
-        } else {
-            bits = (static_cast<uint64_t>(biased - 1) << 52) + mm;
-            if (bits >= 0x7FF0000000000000ull) bits = 0x7FF0000000000000ull;
-        }
-    } else {
-        bits = mm;
+    // the magnitude's floor: -(S + f) = ~S + (1 - f) when f != 0
+    unsigned __int128 m = static_cast<unsigned __int128>(S);
+    if (neg) m = ~m + (sticky ? 0u : 1u);
+    unsigned long long hi = static_cast<unsigned long long>(m >> 64), lo = static_cast<unsigned long long>(m);
+    if ((hi | lo) == 0) return 0ull;
+    // normalise: the top bit of m to bit 63 of hi, what falls below into its lowest bit
+    int L = 128;
+    if (hi == 0) {
+        hi = lo;
+        lo = 0;
+        L = 64;
     }
-    if (neg) bits |= 0x8000000000000000ull;
-    return __longlong_as_double(static_cast<long long>(bits));
+    const int n = clz64(hi);
+    L -= n;
+    hi = (hi << n) | ((lo >> 1) >> (63 - n));
+    if ((lo << n) != 0 || sticky) hi |= 1ull;
+    const unsigned long long sign = neg ? 0x8000000000000000ull : 0ull;
+    const int biased = L + e2 + 1022;
+    if (mode == OUT_RZ_REF)
+        return (hi >> 11) - 0x0010000000000000ull + sign + (static_cast<unsigned long long>(static_cast<long long>(biased)) << 52);
+    if (biased < 1 || biased > 2046) return sign | round_out_of_range(hi, biased);
+    const uint32_t w = static_cast<uint32_t>(hi);
+    const uint32_t up = ((w & 0x7FFu) + 0x3FFu + ((w >> 11) & 1u)) >> 11;
+    return sign + (static_cast<unsigned long long>(biased - 1) << 52) + (hi >> 11) + up;
 }
 
 // ------------------------------------------------------------ drain schedule
 // Block g is drained after chunk c when (c + 1 + blk_off[g]) % blk_period[g] == 0,
-// and every block after the last chunk.  The MMA issuer and the drain warps step
-// identical copies of this schedule.
+// and every block after the last chunk.  The issuing warps step copies of this
+// schedule, the first drain warp the same one lane per block.
 struct DrainSchedule {
-    int r[kMaxGroups];
+    int r[kMaxGroups];  // chunks until each block's next drain, counted from the last event
+    int span, till;     // chunks from the last event to the next, and still to go
     __device__ __forceinline__ void init(const GemmArgs &g) {
+        span = 1 << 30;
 #pragma unroll
-        for (int i = 0; i < kMaxGroups; ++i) r[i] = (i < g.G) ? (1 + g.blk_off[i]) % g.blk_period[i] : 1;
+        for (int i = 0; i < kMaxGroups; ++i)
+            if (i < g.G) {
+                r[i] = g.blk_first[i];
+                span = min(span, r[i]);
+            }
+        till = span;
     }
     // Mask of the blocks drained after the current chunk; advances to the next chunk.
     __device__ __forceinline__ uint32_t next(const GemmArgs &g, bool last) {
         uint32_t m = 0;
+        if (--till == 0) {
+            int nx = 1 << 30;
 #pragma unroll
-        for (int i = 0; i < kMaxGroups; ++i) {
-            if (i < g.G) {
-                if (r[i] == 0) m |= 1u << i;
-                r[i] = (r[i] + 1 == g.blk_period[i]) ? 0 : r[i] + 1;
-            }
+            for (int i = 0; i < kMaxGroups; ++i)
+                if (i < g.G) {
+                    r[i] -= span;
+                    if (r[i] == 0) {
+                        m |= 1u << i;
+                        r[i] = g.blk_period[i];
+                    }
+                    nx = min(nx, r[i]);
+                }
+            span = till = nx;
         }
         return last ? ((1u << g.G) - 1u) : m;
     }
@@ -373,9 +315,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     constexpr int PARTS = kEpiWarps / 4;          // drain warps sharing one TMEM lane quadrant
     constexpr int COLS = BN / PARTS;              // columns per drain thread
     constexpr int NA = W > 2 ? W - 1 : 1;         // 64-bit accumulator groups per column
-    constexpr int DB = drain_batch(COLS, 2 * NA * COLS);
     static_assert(NA <= kMaxAcc, "accumulator groups");
-    static_assert(COLS % 4 == 0 && COLS % DB == 0, "BN must split into 4-column parts");
+    static_assert(COLS % 4 == 0, "BN must split into 4-column parts");
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -384,58 +325,70 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     uint64_t *gfull = empty + g.stages;
     uint64_t *gempty = gfull + 2 * kMaxGroups;  // [block][buffer]: index 2 * blk + buf
     uint64_t *mma_done = gempty + 2 * kMaxGroups;
-    uint64_t *split_bar = mma_done + 1;  // the drain warps' barrier around a split tile's count
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(split_bar + 1);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
     volatile int *vabort = abort_flag;
-    // the drain warps' block table: TMEM column of bin lo of block g in buffer b
-    // at [2 g + b], then lo at [2 kMaxGroups + g] and nb at [3 kMaxGroups + g]
-    int *drn = abort_flag + 1;
-    int *split_flag = drn + 4 * kMaxGroups;  // this CTA's part completed a split tile
+    // accumulator group of bin j and the log2 of its weight in it: a | rel << 8 at [j]
+    int *bin_tab = abort_flag + 1;
+    int *split_flag = bin_tab + 32;  // this CTA's part completed a split tile
+    // the drain warps' last two commands
+    int2 *drain_cmd = reinterpret_cast<int2 *>((reinterpret_cast<uintptr_t>(split_flag + 1) + 7) & ~uintptr_t(7));
+    // the issuers' UMMA lists, decoded: x = accumulator column | the block's other
+    // buffer's << 16, y = A offset | block << 16 | entries left in the block << 24,
+    // z = B offset (descriptor units), w = instruction descriptor
+    uint4 *recs = reinterpret_cast<uint4 *>((reinterpret_cast<uintptr_t>(drain_cmd + 2) + 15) & ~uintptr_t(15));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    // zero B slices below and above the loaded ones (read by out-of-range pairs)
-    {
-        const uint32_t pad_hi_bytes = g.b_region_bytes - g.b_pad_lo_bytes - g.b_block_bytes;
-        for (int st = 0; st < g.stages; ++st) {
-            uint8_t *breg = smem + static_cast<size_t>(st) * g.stage_bytes + g.a_block_bytes;
-            for (uint32_t i = threadIdx.x * 16; i < g.b_pad_lo_bytes; i += kThreads * 16)
-                *reinterpret_cast<uint4 *>(breg + i) = make_uint4(0, 0, 0, 0);
-            uint8_t *top = breg + g.b_pad_lo_bytes + g.b_block_bytes;
-            for (uint32_t i = threadIdx.x * 16; i < pad_hi_bytes; i += kThreads * 16)
-                *reinterpret_cast<uint4 *>(top + i) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
     const int n_iss = g.n_iss < 1 ? 1 : (g.n_iss > kMaxIssuers ? kMaxIssuers : g.n_iss);  // MMA-issuing warps
+    for (int i = threadIdx.x; i < g.op_end[n_iss - 1]; i += kThreads) {
+        const uint32_t op = g.ops[i];
+        const int p = op_p(op), lo = op_lo(op), nb = op_nb(op);
+        auto block_of = [&](int bin) {
+            int b = 0;
+            for (int x = 1; x < g.G; ++x) b += bin >= g.blk_lo[x] ? 1 : 0;
+            return b;
+        };
+        const int blk = block_of(lo);
+        int count = 1;  // entries of the block from this one on
+        while (i + count < g.op_end[n_iss - 1] && block_of(op_lo(g.ops[i + count])) == blk) ++count;
+        const uint32_t d0 = static_cast<uint32_t>(lo * BN);
+        const uint32_t d1 = ((g.dbl_mask >> blk) & 1u)
+                                ? static_cast<uint32_t>(g.blk_col1[blk] + (lo - g.blk_lo[blk]) * BN)
+                                : d0;
+        const uint32_t idesc = (F8 ? idesc_e4m3_f32(BM, 16) : idesc_bf16_f32(BM, 16)) & ~(0x3Fu << 17);
+        recs[i] = make_uint4(d0 | (d1 << 16),
+                             static_cast<uint32_t>(p) * ((BM * KC * 2) >> 4) | (static_cast<uint32_t>(blk) << 16) |
+                                 (static_cast<uint32_t>(count) << 24),
+                             static_cast<uint32_t>(lo - p) * ((BN * KC * 2) >> 4),
+                             idesc | (static_cast<uint32_t>((nb * BN) >> 3) << 17));
+    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < g.stages; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], n_iss);
         }
-        // a block's drain waits for every issuer that has runs in it: its runs are
-        // consecutive run numbers, so min(runs, n_iss) issuers
         for (int i = 0; i < g.G; ++i) {
-            const int runs = g.blk_p1[i] - g.blk_p0[i] + 1;
-            const int contributors = runs < n_iss ? runs : n_iss;
             for (int b = 0; b < 2; ++b) {
-                mbar_init(&gfull[2 * i + b], contributors);
+                mbar_init(&gfull[2 * i + b], 1);
                 mbar_init(&gempty[2 * i + b], kEpiWarps);
             }
         }
         mbar_init(mma_done, n_iss);
-        mbar_init(split_bar, kEpiWarps);
-        for (int i = 0; i < g.G; ++i) {
-            drn[2 * i] = g.blk_lo[i] * BN;
-            drn[2 * i + 1] = ((g.dbl_mask >> i) & 1u) ? g.blk_col1[i] : g.blk_lo[i] * BN;
-            drn[2 * kMaxGroups + i] = g.blk_lo[i];
-            drn[3 * kMaxGroups + i] = g.blk_nb[i];
-        }
         *abort_flag = (*reinterpret_cast<volatile int *>(g.err) != 0) ? 1 : 0;
         fence_mbar_init();
     }
-    if (warp == 1) {
+    if (warp == 1 && lane < g.J) {
+        const int tb = g.J - 1 - lane;
+        int a = 0, t0 = 0;
+        for (int y = 1; y < g.n_acc; ++y)
+            if (tb >= g.acc_t0[y]) {
+                a = y;
+                t0 = g.acc_t0[y];
+            }
+        bin_tab[lane] = a | (g.b * (tb - t0)) << 8;
+    }
+    if (warp == 0) {
         tmem_alloc(tmem_slot, g.tmem_cols);
         tmem_relinquish();
     }
@@ -444,19 +397,23 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint64_t TO = g.timeout_ns;
-    // Every UMMA accumulates, so TMEM starts zeroed (and each drain leaves what it
-    // read zeroed): drain warp (quadrant qd, part) clears its quarter of the columns.
-    if (warp >= 2 && warp < 2 + kEpiWarps) {
+    if (g.zero_mask && warp >= kCtrlWarps) {
+        // blocks whose UMMAs always accumulate start zeroed
         const uint32_t quarter = g.tmem_cols >> 2;
-        const uint32_t base = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + ((warp - 2) >> 2) * quarter;
+        const uint32_t base =
+            tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + ((warp - kCtrlWarps) >> 2) * quarter;
         for (uint32_t col = 0; col < quarter; col += 8) tmem_st8_zero(base + col);
         tmem_st_wait();
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    if (g.zero_mask) {
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
 
-    if (warp == 0) {
+    if (warp < kCtrlWarps) {
+      regs_dec<kCtrlRegs>();
+      if (warp == 0) {
         // ------------------------------------------------------ producer
         if (lane == 0) {
             long long issued = 0;  // stage uses by this CTA over all of its tiles
@@ -484,8 +441,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                     uint8_t *dst = smem + static_cast<size_t>(st) * g.stage_bytes;
                     mbar_arrive_expect_tx(&full[st], g.a_block_bytes + g.b_block_bytes);
                     bulk_g2s(dst, tr.a_src + static_cast<size_t>(c) * g.a_block_bytes, g.a_block_bytes, &full[st]);
-                    bulk_g2s(dst + g.a_block_bytes + g.b_pad_lo_bytes,
-                             tr.b_src + static_cast<size_t>(c) * g.b_block_bytes, g.b_block_bytes, &full[st]);
+                    bulk_g2s(dst + g.a_block_bytes, tr.b_src + static_cast<size_t>(c) * g.b_block_bytes, g.b_block_bytes,
+                             &full[st]);
                     ++issued;
                     if (++st == g.stages) st = 0;
                 }
@@ -496,51 +453,32 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
             for (long long c = (first > 0 ? first : 0); c < issued; ++c)
                 mbar_wait(&full[c % g.stages], static_cast<uint32_t>((c / g.stages) & 1), &zero, TO);
         }
-    } else if (warp == 1 || warp >= kIssuer2Warp) {
+      } else {
         // ---------------------------------------------------- MMA issuers
-        // Up to three issuing warps (on different SM sub-partitions), each run warp-wide
-        // with lane 0 issuing and committing.  The UMMA runs of a K step (block g,
-        // A slice p: ksteps UMMAs) are numbered block by block and dealt round-robin:
-        // issuer iss takes the runs r with r % n_iss == iss.  Every UMMA accumulates
-        // (the drain warps leave the accumulators they read out zeroed), so the
-        // issuers of one block need no ordering among themselves.
-        const int iss = warp == 1 ? 0 : warp - kIssuer2Warp + 1;
+        // Up to three issuing warps (on different SM sub-partitions).  Each owns some of
+        // the bin blocks and issues all of their UMMAs, so a block's UMMAs run in order:
+        // the first after a drain overwrites the accumulator, and a block that waits for
+        // its drain holds up its own issuer alone, while the others go on to the chunks
+        // that the stage ring holds.  What the warp executes per UMMA decides its rate
+        // (it shares its scheduler with four drain warps): four entries at a time, so
+        // that their loads and descriptor arithmetic overlap, run warp-wide with one
+        // elected lane issuing (55 cycles a UMMA with nothing else on the SM, 77 in a
+        // branch of lane 0; one entry at a time 190 to 230 in this kernel).
+        const int iss = warp - 1;
         if (iss < n_iss) {
-            constexpr uint32_t a_step = (BM * KC * 2) >> 4;  // descriptor units (16 B)
-            constexpr uint32_t b_step = (BN * KC * 2) >> 4;
-            constexpr uint32_t sbo = KC * 16;
             constexpr int ksteps = KC >> 4;
+            constexpr uint32_t sbo = KC * 16;
+            // descriptors of stage 0's A and B; the address is in the low word, and
+            // adding offsets never carries out of its 14 bits
             const uint32_t a0 = smem_u32(smem);
-            const uint64_t ad0 = smem_desc(a0, 128, sbo);
-            const uint64_t bd0 = smem_desc(a0 + g.a_block_bytes + g.b_pad_lo_bytes, 128, sbo);
-            const uint32_t idesc_base = (F8 ? idesc_e4m3_f32(BM, 16) : idesc_bf16_f32(BM, 16)) & ~(0x3Fu << 17);
-            // block table in the lanes (lane i: block i): bins, A slices, second buffer,
-            // and this issuer's first A slice in the block (> p1: no runs there)
-            int t_lo = 0, t_nb = 0, t_p0 = 0, t_p1 = -1, t_c1 = 0;
-#pragma unroll
-            for (int i = 0; i < kMaxGroups; ++i)
-                if (lane == i && i < g.G) {
-                    t_lo = g.blk_lo[i];
-                    t_nb = g.blk_nb[i];
-                    t_p0 = g.blk_p0[i];
-                    t_p1 = g.blk_p1[i];
-                    t_c1 = g.blk_col1[i];
-                }
-            const int runs = t_p1 - t_p0 + 1;
-            int incl = runs;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, off);
-                if (lane >= off) incl += y;
-            }
-            const int rb = incl - runs;  // runs of the blocks before this one
-            const int t_pf = t_p0 + ((iss - rb % n_iss) % n_iss + n_iss) % n_iss;
-            const uint32_t mine = __ballot_sync(0xffffffffu, lane < g.G && t_pf <= t_p1);
-            const uint32_t dbl = g.dbl_mask & mine;  // double-buffered: UMMAs go on during their drains
-            uint32_t ephase = 0;  // parity of the gempty waits, bit 2 blk + buf
-            uint32_t pend = 0;    // drains committed and not yet waited for, bit 2 blk + buf
-            uint32_t bufm = 0;    // accumulator buffer each block writes now
-            uint32_t prev = 0;    // single-buffered blocks drained after the previous chunk
+            const uint64_t ad0 = smem_desc(a0, 128, sbo), bd0 = smem_desc(a0 + g.a_block_bytes, 128, sbo);
+            const uint32_t a_lo = static_cast<uint32_t>(ad0), b_lo = static_cast<uint32_t>(bd0);
+            const uint64_t d_hi = ad0 & 0xFFFFFFFF00000000ull;
+            const int r0 = iss ? g.op_end[iss - 1] : 0, r1 = g.op_end[iss];
+            uint32_t ephase = 0;   // parity of the gempty waits, bit 2 blk + buf
+            uint32_t pend = 0;     // drains committed and not yet waited for, bit 2 blk + buf
+            uint32_t bufm = 0;     // accumulator buffer each block writes now
+            uint32_t fresh = ~0u;  // blocks whose next UMMA is the first after a drain
             int st = 0;
             uint32_t fparity = 0;
             bool ok = true;
@@ -551,76 +489,75 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                 ds.init(g);
                 for (int c = tr.c0; c < tr.c1; ++c) {
                     const uint32_t cur = ds.next(g, c == tr.c1 - 1);
-                    int got = 1;
-                    if (lane == 0) got = mbar_wait(&full[st], fparity, vabort, TO) ? 1 : 0;
-                    if (!__shfl_sync(0xffffffffu, got, 0)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[st], fparity, vabort, TO))) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t stage_off = (static_cast<uint64_t>(st) * g.stage_bytes) >> 4;
-                    // issue order: blocks drained after this chunk, then the rest, then the
-                    // blocks whose drain (after the previous chunk) must finish first
-                    const uint32_t order[3] = {cur & mine & ~prev, mine & ~cur & ~prev, prev};
-                    for (int cls = 0; ok && cls < 3; ++cls) {
-                        uint32_t m = order[cls];
-                        while (m) {
-                            const int blk = __ffs(m) - 1;
-                            const uint32_t bit = 1u << blk;
-                            m &= m - 1;
-                            const int lo = __shfl_sync(0xffffffffu, t_lo, blk);
-                            const int nb = __shfl_sync(0xffffffffu, t_nb, blk);
-                            const int p1 = __shfl_sync(0xffffffffu, t_p1, blk);
-                            const int pf = __shfl_sync(0xffffffffu, t_pf, blk);
-                            const int c1 = __shfl_sync(0xffffffffu, t_c1, blk);
-                            const int bb = static_cast<int>((bufm >> blk) & 1u);
-                            const int ix = 2 * blk + bb;
-                            if ((pend >> ix) & 1u) {
-                                // the buffer's previous drain must have read it out
-                                int gote = 1;
-                                if (lane == 0) gote = mbar_wait(&gempty[ix], (ephase >> ix) & 1u, vabort, TO) ? 1 : 0;
-                                if (!__shfl_sync(0xffffffffu, gote, 0)) {
-                                    ok = false;
-                                    break;
-                                }
-                                ephase ^= 1u << ix;
-                                pend &= ~(1u << ix);
-                                tc_fence_after();
-                            }
-                            const uint32_t d_tmem = tmem + static_cast<uint32_t>(bb ? c1 : lo * BN);
-                            const uint32_t idesc = idesc_base | (static_cast<uint32_t>((nb * BN) >> 3) << 17);
-                            for (int p = pf; p <= p1; p += n_iss) {
-                                // A slice p against B slices q = j - p of the block's bins j
-                                const uint64_t ad = ad0 + stage_off + static_cast<uint64_t>(p) * a_step;
-                                const uint64_t bd =
-                                    bd0 + stage_off + static_cast<uint64_t>(static_cast<int64_t>(lo - p) * b_step);
-                                if (lane == 0) {
+                    const uint32_t soff = (static_cast<uint32_t>(st) * g.stage_bytes) >> 4;
+                    for (int i = r0; i < r1;) {
+                        // one block: its list ends where the first entry's count says
+                        uint4 rc[4];
 #pragma unroll
-                                    for (int kk = 0; kk < ksteps; ++kk) {
-                                        // one UMMA covers 32 bytes of K per row: 16 bf16 or 32 e4m3 values
-                                        if constexpr (F8)
-                                            umma_e4m3(d_tmem, ad + static_cast<uint64_t>(kk * 16),
-                                                      bd + static_cast<uint64_t>(kk * 16), idesc, 1u);
-                                        else
-                                            umma_bf16(d_tmem, ad + static_cast<uint64_t>(kk * 16),
-                                                      bd + static_cast<uint64_t>(kk * 16), idesc, 1u);
+                        for (int x = 0; x < 4; ++x) rc[x] = recs[min(i + x, r1 - 1)];
+                        const uint32_t blk = (rc[0].y >> 16) & 0xFu;
+                        const int end = i + static_cast<int>(rc[0].y >> 24);
+                        const uint32_t buf = (bufm >> blk) & 1u, ix = 2 * blk + buf;
+                        if ((pend >> ix) & 1u) {
+                            // the buffer's previous drain must have read it out
+                            if (!__all_sync(0xffffffffu, mbar_wait(&gempty[ix], (ephase >> ix) & 1u, vabort, TO))) {
+                                ok = false;
+                                break;
+                            }
+                            ephase ^= 1u << ix;
+                            pend &= ~(1u << ix);
+                            tc_fence_after();
+                        }
+                        // a drained block's first UMMA spans the block and overwrites it
+                        uint32_t acc0 = ((fresh & ~g.zero_mask) >> blk & 1u) ^ 1u;
+                        fresh &= ~(1u << blk);
+                        while (true) {
+                            if (elect_one()) {
+#pragma unroll
+                                for (int x = 0; x < 4; ++x) {
+                                    const uint32_t d = tmem + (buf ? rc[x].x >> 16 : rc[x].x & 0xFFFFu);
+                                    const uint64_t ad = d_hi | (a_lo + soff + (rc[x].y & 0xFFFFu));
+                                    const uint64_t bd = d_hi | (b_lo + soff + rc[x].z);
+                                    if (x == 0 || i + x < end) {
+#pragma unroll
+                                        for (int kk = 0; kk < ksteps; ++kk) {
+                                            // one UMMA covers 32 bytes of K per row: 16 bf16 or 32 e4m3 values
+                                            const uint32_t acc = x == 0 && kk == 0 ? acc0 : 1u;
+                                            if constexpr (F8)
+                                                umma_e4m3(d, ad + kk * 16, bd + kk * 16, rc[x].w, acc);
+                                            else
+                                                umma_bf16(d, ad + kk * 16, bd + kk * 16, rc[x].w, acc);
+                                        }
                                     }
                                 }
                             }
-                            if (cur & bit) {
-                                if (lane == 0) umma_commit(&gfull[ix]);
-                                pend |= 1u << ix;
-                                if (dbl & bit) bufm ^= bit;
-                            }
+                            __syncwarp();
+                            acc0 = 1u;
+                            i = min(i + 4, end);
+                            if (i == end) break;
+#pragma unroll
+                            for (int x = 0; x < 4; ++x) rc[x] = recs[min(i + x, r1 - 1)];
+                        }
+                        if ((cur >> blk) & 1u) {
+                            if (elect_one()) umma_commit(&gfull[ix]);
+                            __syncwarp();
+                            pend |= 1u << ix;
+                            bufm ^= g.dbl_mask & (1u << blk);
+                            fresh |= 1u << blk;
                         }
                     }
                     if (!ok) break;
-                    if (lane == 0) umma_commit(&empty[st]);
+                    if (elect_one()) umma_commit(&empty[st]);
+                    __syncwarp();
                     if (++st == g.stages) {
                         st = 0;
                         fparity ^= 1u;
                     }
-                    prev = cur & mine & ~dbl;
                 }
             }
             if (!ok && lane == 0 && !*vabort) {
@@ -628,101 +565,112 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                 *vabort = 1;
             }
             // all MMAs issued by this warp complete before TMEM is released
-            if (lane == 0) {
-                umma_commit(mma_done);
-                const int zero = 0;
-                mbar_wait(mma_done, 0, &zero, TO);
-            }
+            if (elect_one()) umma_commit(mma_done);
+            __syncwarp();
+            const int zero = 0;
+            mbar_wait(mma_done, 0, &zero, TO);
         }
-        __syncwarp();
+      }
+      __syncwarp();
     } else {
         // ------------------------------------------ drain + epilogue warps
-        const int ew = warp - 2;
+        regs_inc<kDrainRegs>();
+        const int ew = warp - kCtrlWarps;
         const int qd = warp & 3;  // TMEM lane quadrant accessible to this warp
         const int part = ew >> 2;  // which COLS-wide column slice of the tile
         const uint32_t trow = tmem + (static_cast<uint32_t>(32 * qd) << 16) + static_cast<uint32_t>(part * COLS);
 
         long long acc[COLS][NA];
+        // The first drain warp steps the drain schedule, waits for each drain's UMMAs (a
+        // bounded wait) and passes the others a command through shared memory: x the
+        // TMEM column of the buffer less lo BN, y = lo | hi << 8 | zero it << 16 | end of the
+        // tile << 17 | gempty index << 20, or -1 when the wait gave up.  They wait at
+        // a hardware barrier.  (Sixteen warps stepping the schedule and waiting on the
+        // mbarrier took issue slots that the MMA-issuing warps of their schedulers
+        // needed.)  One command slot per parity: a slot is written again only after
+        // every warp has passed the barrier in between, so all of them leave at the
+        // same command.
         uint32_t fphase = 0;  // parity of the gfull waits, bit 2 blk + buf
         uint32_t dbuf = 0;    // accumulator buffer each block's next drain reads
-        uint32_t prev = 0;
+        uint32_t n_cmd = 0;
         bool ok = true;
-        // barrier of the 16 drain warps (one arrival per warp), with the bounded wait
-        // of every other barrier: a warp that gave up cannot leave the others waiting
-        uint32_t sphase = 0;
-        auto drain_bar = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(split_bar);
-            const bool got = mbar_wait(split_bar, sphase, vabort, TO);
-            sphase ^= 1u;
-            return got;
-        };
         for (int t = g.tile_begin + static_cast<int>(blockIdx.x); ok && t < g.total_tiles; t += gridDim.x) {
-            TileRef tr;
-            tile_ref(g, t, &tr);
 #pragma unroll
             for (int i = 0; i < COLS; ++i)
 #pragma unroll
                 for (int a = 0; a < NA; ++a) acc[i][a] = 0;
-
-            DrainSchedule ds;
-            ds.init(g);
-            for (int c = tr.c0; ok && c < tr.c1; ++c) {
-                const bool last = (c == tr.c1 - 1);
-                const uint32_t cur = ds.next(g, last);
-                for (int pass = 0; ok && pass < 2; ++pass) {
-                    uint32_t m = pass == 0 ? (cur & ~prev) : (cur & prev);
-                    while (m) {
-                        const int blk = __ffs(m) - 1;
-                        m &= m - 1;
-                        const int bb = static_cast<int>((dbuf >> blk) & 1u);
-                        const int ix = 2 * blk + bb;
-                        const bool gotg = mbar_wait(&gfull[ix], (fphase >> ix) & 1u, vabort, TO);
-                        if (!gotg) {
-                            ok = false;
-                            break;
-                        }
-                        fphase ^= 1u << ix;
-                        tc_fence_after();
-                        const int lo = drn[2 * kMaxGroups + blk];
-                        const int hi = lo + drn[3 * kMaxGroups + blk] - 1;
-                        // bin j of the buffer read is at column drn[ix] + (j - lo) BN
-                        const uint32_t bbase = trow + static_cast<uint32_t>(drn[ix] - lo * BN);
-                        for (int j = lo; j <= hi; ++j) {
-                            // accumulator group of bin j and its weight within the group
-                            const int t = g.J - 1 - j;
-                            int a = 0, t0 = 0;
-#pragma unroll
-                            for (int x = 1; x < NA; ++x)
-                                if (x < g.n_acc && t >= g.acc_t0[x]) {
-                                    a = x;
-                                    t0 = g.acc_t0[x];
-                                }
-                            const int rel = g.b * (t - t0);
-#pragma unroll
-                            for (int cb = 0; cb < COLS / DB; ++cb) {
-                                uint32_t v[DB];
-                                const uint32_t taddr = bbase + static_cast<uint32_t>(j * BN + cb * DB);
-                                tmem_ld_cols<DB>(taddr, v);
-                                tmem_ld_wait();
-                                tmem_zero_cols<DB>(taddr);  // the next UMMAs accumulate onto zero
-#pragma unroll
-                                for (int i = 0; i < DB; ++i) reg_fence(v[i]);
-                                acc_add_group<NA, DB>(acc + cb * DB, v, a, rel);
-                            }
-                        }
-                        // the buffer is zeroed and free for the block's UMMAs again
+            // the first warp's schedule: lane i counts the chunks to block i's next drain
+            int left = 0, until = 1 << 30;
+            uint32_t m = 0;  // blocks still to drain at this point
+            if (ew == 0) {
+                TileRef tr;
+                tile_ref(g, t, &tr);
+                left = tr.c1 - tr.c0;
+                if (lane < g.G) until = g.blk_first[lane];
+            }
+            for (bool end = false; !end;) {
+                if (ew == 0) {
+                    if (m == 0) {
+                        const int step = min(__reduce_min_sync(0xffffffffu, until), left);
+                        left -= step;
+                        until -= step;
+                        m = __ballot_sync(0xffffffffu, until == 0 && lane < g.G);
+                        if (until == 0 && lane < g.G) until = g.blk_period[lane];
+                        if (left == 0) m = (1u << g.G) - 1u;
+                    }
+                    const int blk = __ffs(m) - 1;
+                    m &= m - 1;
+                    const int ix = 2 * blk + static_cast<int>((dbuf >> blk) & 1u);
+                    const int blo = g.blk_lo[blk];
+                    const int2 cmd = make_int2(
+                        (ix & 1) ? g.blk_col1[blk] - blo * BN : 0,
+                        blo | (blo + g.blk_nb[blk] - 1) << 8 | static_cast<int>((g.zero_mask >> blk) & 1u) << 16 |
+                            (m == 0 && left == 0 ? 1 << 17 : 0) | ix << 20);
+                    const bool got = mbar_wait(&gfull[ix], (fphase >> ix) & 1u, vabort, TO);
+                    fphase ^= 1u << ix;
+                    dbuf ^= g.dbl_mask & (1u << blk);
+                    if (lane == 0) drain_cmd[n_cmd & 1] = got ? cmd : make_int2(0, -1);
+                    tc_fence_before();
+                }
+                named_barrier<1, 32 * kEpiWarps>();
+                tc_fence_after();
+                const int2 cmd = drain_cmd[n_cmd++ & 1];
+                if (cmd.y < 0) {
+                    ok = false;
+                    break;
+                }
+                end = ((cmd.y >> 17) & 1) != 0;
+                const int lo = cmd.y & 0xFF, hi = (cmd.y >> 8) & 0xFF;
+                const uint32_t bbase = trow + static_cast<uint32_t>(cmd.x);  // bin j at bbase + j BN
+                // One bin at a time (several at once, for overlapped loads, cost more in
+                // registers and code: 3.86 against 3.67 ms at 4096^3, s = 8, p + q <= 8); after
+                // the last bin's load the buffer is free, so that its conversion overlaps the
+                // block's next UMMAs.
+#pragma unroll 1
+                for (int j = lo; j <= hi; ++j) {
+                    uint32_t v[COLS];
+                    const uint32_t taddr = bbase + static_cast<uint32_t>(j * BN);
+                    tmem_ld_cols<COLS>(taddr, v);
+                    const int bt = bin_tab[j];
+                    tmem_ld_wait();
+                    if ((cmd.y >> 16) & 1) {
+                        tmem_zero_cols<COLS>(taddr);
                         tmem_st_wait();
+                    }
+                    if (j == hi) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&gempty[ix]);
-                        if ((g.dbl_mask >> blk) & 1u) dbuf ^= 1u << blk;
+                        if (lane == 0) mbar_arrive(&gempty[cmd.y >> 20]);
                     }
+#pragma unroll
+                    for (int i = 0; i < COLS; ++i) reg_fence(v[i]);
+                    acc_add_group<NA, COLS>(acc, v, bt & 0xFF, bt >> 8);
                 }
-                prev = cur & ~g.dbl_mask;
             }
             if (!ok) break;
 
+            TileRef tr;
+            tile_ref(g, t, &tr);
             if (tr.split >= 0) {
                 // a part of a split tile: add the exact group sums into the tile's
                 // scratch (integer adds, exact in any order); the part that completes
@@ -737,16 +685,10 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                             atomicAdd(sa + (static_cast<size_t>(a) * BN + part * COLS + i) * BM + rl,
                                       static_cast<unsigned long long>(acc[i][a]));
                 __threadfence();
-                if (!drain_bar()) {
-                    ok = false;
-                    break;
-                }
+                named_barrier<1, 32 * kEpiWarps>();
                 if (ew == 0 && lane == 0)
                     *split_flag = (atomicAdd(g.split_cnt + tr.split, 1) == g.split_parts - 1) ? 1 : 0;
-                if (!drain_bar()) {
-                    ok = false;
-                    break;
-                }
+                named_barrier<1, 32 * kEpiWarps>();
                 if (!*reinterpret_cast<volatile int *>(split_flag)) continue;
                 __threadfence();
                 // the totals, leaving the scratch zero for the next launch
@@ -768,21 +710,9 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
             const int row = tr.mt * BM + 32 * qd + lane;
             const int col0 = tr.nt * BN + part * COLS;
             if (row < tr.M) {
-                // the scale exponents first, as independent loads, so that their
-                // latency is paid once rather than once per column
                 const int er = __ldg(tr.er + row);
-                int es[COLS];
-#pragma unroll
-                for (int i = 0; i < COLS; ++i) es[i] = er + (col0 + i < tr.N ? __ldg(tr.ec + col0 + i) : 0);
-                const int bJ1 = g.b * (g.J + 1);
-                // the exact sum of column i: sum_a acc[i][a] 2^(b acc_t0[a]) in W words
-                auto exact_q = [&](int i, uint32_t (&q)[W]) {
-#pragma unroll
-                    for (int w = 0; w < W; ++w) q[w] = 0;
-#pragma unroll
-                    for (int x = 0; x < NA; ++x)
-                        if (x < g.n_acc) q_add_i64<W>(q, acc[i][x], g.b * g.acc_t0[x]);
-                };
+                auto scale_of = [&](int i) { return er + (i < COLS && col0 + i < tr.N ? __ldg(tr.ec + col0 + i) : 0); };
+                const int e_base = -2044 - g.b * (g.J + 1);
                 if (g.out_mode == OUT_PAIRS) {
                     // the reference's device output: lo, then hi with bits 51..62 = Er + Ec
 #pragma unroll
@@ -795,7 +725,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                             unsigned long long hi = 0;
                             if constexpr (NA > 1) hi = g.n_acc > 1 ? static_cast<unsigned long long>(acc[i][1]) : 0ull;
                             const unsigned long long scale =
-                                static_cast<unsigned long long>(static_cast<uint32_t>(es[i]));
+                                static_cast<unsigned long long>(static_cast<uint32_t>(scale_of(i)));
                             hi = (hi & 0x8007FFFFFFFFFFFFull) | ((scale & 0xFFFull) << 51);
                             dst[0] = static_cast<long long>(lo);
                             dst[1] = static_cast<long long>(hi);
@@ -806,12 +736,16 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                     for (int i = 0; i < COLS; ++i) {
                         const int col = col0 + i;
                         if (col < tr.N) {
-                            uint32_t q[W];
-                            exact_q(i, q);
-                            int32_t *dst = g.raw + (static_cast<size_t>(row) * tr.N + col) * 4;
-                            const uint32_t ext = static_cast<uint32_t>(static_cast<int32_t>(q[W - 1]) >> 31);
+                            // the exact sum modulo 2^128
+                            unsigned __int128 q = 0;
 #pragma unroll
-                            for (int w = 0; w < 4; ++w) dst[w] = static_cast<int32_t>(w < W ? q[w] : ext);
+                            for (int x = 0; x < NA; ++x)
+                                if (x < g.n_acc && g.b * g.acc_t0[x] < 128)
+                                    q += static_cast<unsigned __int128>(static_cast<__int128>(acc[i][x]))
+                                         << (g.b * g.acc_t0[x]);
+                            int32_t *dst = g.raw + (static_cast<size_t>(row) * tr.N + col) * 4;
+#pragma unroll
+                            for (int w = 0; w < 4; ++w) dst[w] = static_cast<int32_t>(q >> (32 * w));
                         }
                     }
                 } else {
@@ -820,27 +754,28 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                     // pairs of columns as one 16-byte store where aligned (fewer, larger
                     // writes, which matters most when C is host memory)
                     const bool vec = (reinterpret_cast<uintptr_t>(crow + col0) & 15) == 0;
-                    // at most two accumulator groups, the second at most 63 bits up: the
-                    // 128-bit rounding path
-                    const int B1 = g.n_acc > 1 ? g.b * g.acc_t0[1] : 0;
-                    const bool two_groups = g.out_mode == OUT_RN && g.n_acc <= 2 && B1 <= 63;
+                    int B[kMaxAcc];
+#pragma unroll
+                    for (int x = 0; x < kMaxAcc; ++x) B[x] = g.b * g.acc_t0[x];
+                    // the next pair's scale exponents are loaded a step ahead
+                    int es_next[2] = {scale_of(0), scale_of(1)};
 #pragma unroll
                     for (int i = 0; i < COLS; i += 2) {
+                        const int es[2] = {es_next[0], es_next[1]};
+                        es_next[0] = scale_of(i + 2);
+                        es_next[1] = scale_of(i + 3);
                         double v[2];
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int col = col0 + i + u;
                             v[u] = 0.0;
                             if (col < tr.N) {
-                                if (two_groups) {
-                                    long long a1 = 0;
-                                    if constexpr (NA > 1) a1 = g.n_acc > 1 ? acc[i + u][1] : 0ll;
-                                    v[u] = acc2_to_double_rn(acc[i + u][0], a1, B1, es[i + u], bJ1);
-                                } else {
-                                    uint32_t q[W];
-                                    exact_q(i + u, q);
-                                    v[u] = q_to_double<W>(q, es[i + u], bJ1, g.out_mode);
-                                }
+                                __int128 S;
+                                bool sticky;
+                                int low;
+                                acc_window<NA>(acc[i + u], g.n_acc, B, &S, &sticky, &low);
+                                v[u] = __longlong_as_double(static_cast<long long>(
+                                    window_bits(S, sticky, es[u] + e_base + low, g.out_mode)));
                                 // BLAS semantics: C is not read when beta == 0
                                 if (!plain)
                                     v[u] = g.beta == 0.0 ? g.alpha * v[u] : fma(g.beta, crow[col], g.alpha * v[u]);
@@ -864,7 +799,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     }
 
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem, g.tmem_cols);
     }
@@ -895,17 +830,22 @@ void launch_gemm_variant(const GemmArgs &args, int tiles, size_t smem, void *str
     static std::atomic<bool> raised[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
+    int threads = kThreads;
     if (dev < 0 || dev >= 64 || !raised[dev].load(std::memory_order_acquire)) {
+        // a kernel built with fewer registers than its split hands out would wait for
+        // them forever: refused here as an invalid launch
+        cudaFuncAttributes fa{};
+        if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs < kLaunchRegs) threads = 0;
         int opt = 0;
         cudaDeviceGetAttribute(&opt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              opt > static_cast<int>(smem) ? opt : static_cast<int>(smem));
-        if (dev >= 0 && dev < 64) raised[dev].store(true, std::memory_order_release);
+        if (threads && dev >= 0 && dev < 64) raised[dev].store(true, std::memory_order_release);
     }
     const int range = args.total_tiles - args.tile_begin;
     const int grid = range < device_sm_count() ? range : device_sm_count();
     (void)tiles;
-    kern<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(args);
+    kern<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(args);
 }
 
 }  // namespace ozgb

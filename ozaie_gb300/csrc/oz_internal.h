@@ -25,15 +25,26 @@ constexpr int kMaxBins = 64;      // J limit
 constexpr int kMaxGroups = 8;     // drain groups limit
 constexpr int kMaxAcc = 4;        // 64-bit accumulator groups per element (drain)
 constexpr int kEpiWarps = 16;     // drain + epilogue warps: 4 per TMEM lane quadrant
-// warp 0 producer, warp 1 MMA issuer, then the drain warps, then two more MMA
-// issuers, so that the issuing warps sit on three different schedulers: one thread
-// issues a UMMA about every 80-100 SM cycles, while the tensor pipe takes N / 2
-// cycles for one of N columns, so narrow UMMAs need several issuers to keep it
-// busy.  (640 threads keep ptxas's register limit at 96 per thread.)
-constexpr int kThreads = 64 + 32 * kEpiWarps + 64;
-constexpr int kIssuer2Warp = 2 + kEpiWarps;  // issuing warps: 1, kIssuer2Warp and kIssuer2Warp + 1
+// warp 0 producer, warps 1 to 3 MMA issuers (on three different schedulers: one
+// thread issues a UMMA about every 60-80 SM cycles at best, while the tensor pipe
+// takes N / 2 cycles for one of N columns), then the drain warps.
+constexpr int kCtrlWarps = 4;
+constexpr int kThreads = 32 * (kCtrlWarps + kEpiWarps);
+// Registers per thread: 640 threads leave ptxas 96; the drain warps, which hold the
+// 64-bit sums and a batch of drained values, take 104 and the control warps 64
+// (512 x 104 + 128 x 64 = 640 x 96).
+constexpr int kLaunchRegs = 96, kDrainRegs = 104, kCtrlRegs = 64;
+static_assert(32 * kEpiWarps * kDrainRegs + 32 * kCtrlWarps * kCtrlRegs <= kThreads * kLaunchRegs, "register split");
 constexpr int kMaxIssuers = 3;
 constexpr int kMaxAccWords = 5;
+constexpr int kMaxOps = 512;       // UMMA list of a plan (GemmArgs::ops)
+
+// One entry of a plan's UMMA list: A slice p against the B slices of bins
+// [lo, lo + nb), i.e. q = lo - p .. lo + nb - 1 - p, all within [0, s).
+OZ_HD inline uint16_t pack_op(int p, int lo, int nb) { return static_cast<uint16_t>(p | (lo << 6) | ((nb - 1) << 11)); }
+OZ_HD inline int op_p(uint32_t op) { return static_cast<int>(op & 63u); }
+OZ_HD inline int op_lo(uint32_t op) { return static_cast<int>((op >> 6) & 31u); }
+OZ_HD inline int op_nb(uint32_t op) { return static_cast<int>((op >> 11) & 31u) + 1; }
 
 // OUT_PAIRS writes the reference's device output (its C buffer before the host
 // decode): per element int64 lo, hi with (Er + Ec) in bits 51..62 of hi.
@@ -80,20 +91,25 @@ struct GemmArgs {
     int out_mode;
     int tiles_m, tiles_n;
     int stages;
-    // Stage layout: [A: s slices of BM x KC][B region: pad_lo zero slices, the s
-    // loaded B slices, pad_hi zero slices], each B slice BN x KC.
-    uint32_t stage_bytes, a_block_bytes, b_block_bytes, b_pad_lo_bytes, b_region_bytes;
+    // Stage layout: [A: s slices of BM x KC][B: s slices of BN x KC].
+    uint32_t stage_bytes, a_block_bytes, b_block_bytes;
     uint32_t tmem_cols;
     int *err;
     unsigned long long timeout_ns;
-    // Bin blocks (also the drain groups).  Block g holds bins [lo, lo + nb);
-    // every UMMA of the block covers all of its bins (one accumulator range):
-    // A slice p in [p0, p1] against B slices q = j - p, the out-of-range q
-    // reading zero slices.  Block g is drained after chunk c when
-    // (c + 1 + off) % period == 0, and after the last chunk.
+    // Bin blocks, the drain groups.  Block g holds bins [lo, lo + nb) and is
+    // drained after chunk c when (c + 1 + off) % period == 0, and after the last
+    // chunk.
     int G;
-    int blk_lo[kMaxGroups], blk_nb[kMaxGroups], blk_p0[kMaxGroups], blk_p1[kMaxGroups];
+    int blk_lo[kMaxGroups], blk_nb[kMaxGroups];
     int blk_period[kMaxGroups], blk_off[kMaxGroups];
+    int blk_first[kMaxGroups];  // chunks up to and including its first drain
+    // UMMAs of a K step (pack_op): issuer i's are ops[op_end[i - 1], op_end[i]), those
+    // of a block together, first one that spans the block.  Blocks of zero_mask have no
+    // such UMMA (more bins than slices): theirs all accumulate, and the drain warps
+    // store zeros over what they read.
+    int op_end[kMaxIssuers];
+    uint32_t zero_mask;
+    uint16_t ops[kMaxOps];
     // Double-buffered blocks (bit g of dbl_mask): a second accumulator range at
     // TMEM column blk_col1[g]; after each drain the block's UMMAs switch ranges,
     // so they go on while the drain warps read the other one out.
@@ -124,7 +140,7 @@ struct GemmArgs {
     // below 2^63.  OUT_PAIRS: groups {0, pair_g0}, each modulo 2^64.
     int n_acc;
     int acc_t0[kMaxAcc];
-    int n_iss;  // MMA-issuing warps (1 to 3): the UMMA runs of a K step are dealt round-robin
+    int n_iss;  // MMA-issuing warps (1 to 3), each with its own bin blocks
     double alpha, beta;  // C = alpha * (A B) + beta * C for OUT_RN / OUT_RZ_REF (1, 0: plain store)
 };
 

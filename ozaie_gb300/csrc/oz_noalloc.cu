@@ -27,7 +27,6 @@
 // must detect that case uses ozgb_dgemm_device and ozgb_sync instead.
 #include <cuda_runtime.h>
 
-#include <cstring>
 #include <mutex>
 
 #include "oz_gb300.h"
@@ -127,7 +126,7 @@ extern "C" ozgb_status ozgb_dgemm_device_noalloc(int M, int N, int K, const doub
     if (cudaGetLastError() != cudaSuccess) return OZGB_ERR_EXEC;  // a stage (a) or (b) launch
 
     GemmArgs g;
-    std::memset(&g, 0, sizeof g);
+    gemm_args_from_plan(&g, p, OUT_RN, err, 2000000000ull);
     g.a_tiles = at;
     g.b_tiles = bt;
     g.er = er;
@@ -137,39 +136,9 @@ extern "C" ozgb_status ozgb_dgemm_device_noalloc(int M, int N, int K, const doub
     g.M = M;
     g.N = N;
     g.n_kc = p.n_kc;
-    g.KC = p.KC;
-    g.s = p.cfg.s;
-    g.J = p.cfg.J;
-    g.b = p.cfg.b;
-    g.out_mode = OUT_RN;
     g.tiles_m = p.tiles_m;
     g.tiles_n = p.tiles_n;
     g.total_tiles = p.tiles_m * p.tiles_n;
-    g.alpha = 1.0;  // C = A B
-    g.beta = 0.0;
-    g.stages = p.stages;
-    g.stage_bytes = p.stage_bytes;
-    g.a_block_bytes = p.a_block_bytes;
-    g.b_block_bytes = p.b_block_bytes;
-    g.b_pad_lo_bytes = static_cast<uint32_t>(p.pad_lo) * p.b_slice_bytes;
-    g.b_region_bytes = p.b_region_bytes;
-    g.tmem_cols = p.tmem_cols;
-    g.err = err;
-    g.timeout_ns = 2000000000ull;
-    g.n_acc = p.n_acc;
-    g.n_iss = p.n_iss;
-    for (int a = 0; a < kMaxAcc; ++a) g.acc_t0[a] = p.acc_t0[a];
-    g.G = p.G;
-    for (int i = 0; i < p.G; ++i) {
-        g.blk_lo[i] = p.blk_lo[i];
-        g.blk_nb[i] = p.blk_nb[i];
-        g.blk_p0[i] = p.blk_p0[i];
-        g.blk_p1[i] = p.blk_p1[i];
-        g.blk_period[i] = p.blk_period[i];
-        g.blk_off[i] = p.blk_off[i];
-        g.blk_col1[i] = p.blk_col1[i];
-    }
-    g.dbl_mask = p.dbl_mask;
     p.fn(g, p.tiles_m * p.tiles_n, p.smem, st);
     if (cudaGetLastError() != cudaSuccess) return OZGB_ERR_EXEC;  // the slice-pair GEMM launch
     return OZGB_OK;

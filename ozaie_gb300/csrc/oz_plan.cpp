@@ -5,6 +5,7 @@
 #include <functional>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -355,33 +356,101 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
         p.G = hint.groups;
         p.model_cycles_per_kstep = part_cost(p.G, p.blk_lo, p.blk_nb);
     }
-    p.pad_lo = 0;
-    p.pad_hi = 0;
-    p.mma_per_kstep = 0;
+    // zero B slices that UMMAs spanning whole blocks would read below q = 0 and above
+    // q = s - 1: they are part of the stage size that bounds the slices a product may
+    // have (the UMMA lists below need none)
+    int pad_lo = 0, pad_hi = 0;
     for (int g = 0; g < p.G; ++g) {
         const int lo = p.blk_lo[g], hi = lo + p.blk_nb[g] - 1;
-        p.blk_p0[g] = p0_of(lo);
-        p.blk_p1[g] = p1_of(hi);
-        p.mma_per_kstep += p.blk_p1[g] - p.blk_p0[g] + 1;
-        p.pad_lo = std::max(p.pad_lo, p.blk_p1[g] - lo);           // q = lo - p1 >= -pad_lo
-        p.pad_hi = std::max(p.pad_hi, hi - p.blk_p0[g] - (s - 1));  // q = hi - p0 <= s - 1 + pad_hi
+        pad_lo = std::max(pad_lo, p1_of(hi) - lo);
+        pad_hi = std::max(pad_hi, hi - p0_of(lo) - (s - 1));
     }
 
-    // issuing warps (1 to 3; the UMMA runs of a K step are dealt round-robin): one
-    // warp issues a UMMA about every 80-100 SM cycles and the tensor pipe takes
-    // N / 2 cycles for N columns, so three unless there are fewer runs than that
-    p.n_iss = hint.issuers >= 1 && hint.issuers <= kMaxIssuers ? hint.issuers : kMaxIssuers;
-    p.n_iss = std::min(p.n_iss, std::max(1, p.mma_per_kstep));
-
+    // ---- double buffering: blocks get a second accumulator range in the TMEM
+    // columns the bins leave free, most frequently drained blocks first (the
+    // order does not depend on K, so problems of one shape class share a plan);
+    // their UMMAs then switch ranges at each drain, and at the end of a tile,
+    // instead of waiting for the drain warps to read the block out.
+    p.dbl_mask = 0;
+    int next_col = J * p.BN;  // buffer 0: bin j at column j BN
+    if (hint.dbl != 0) {
+        int order[kMaxGroups], n = 0;
+        long period[kMaxGroups];  // in K values, not clamped to this K
+        for (int g = 0; g < p.G; ++g) {
+            order[n++] = g;
+            period[g] = 1L << 40;
+            for (int j = p.blk_lo[g]; j < p.blk_lo[g] + p.blk_nb[g]; ++j)
+                period[g] = std::min(period[g], static_cast<long>(std::floor(16777216.0 / (pairs_in_bin(j, s) * v2 * v2))));
+        }
+        std::sort(order, order + n, [&](int x, int y) {
+            return period[x] != period[y] ? period[x] < period[y] : (p.blk_nb[x] != p.blk_nb[y] ? p.blk_nb[x] > p.blk_nb[y] : x < y);
+        });
+        for (int i = 0; i < n; ++i) {
+            const int g = order[i];
+            if (next_col + p.blk_nb[g] * p.BN > 512) continue;
+            p.dbl_mask |= 1u << g;
+            p.blk_col1[g] = next_col;
+            next_col += p.blk_nb[g] * p.BN;
+        }
+    }
+    uint32_t cols = 32;
+    while (cols < static_cast<uint32_t>(next_col)) cols <<= 1;
+    p.tmem_cols = cols;
+    // ---- UMMA lists.  A UMMA takes A slice p against consecutive B slices, so it
+    // covers consecutive bins of one block; it spans exactly the bins that hold a pair
+    // (p, q) (on GB300 a UMMA of N columns takes max(N / 2, 32 + N / 4) cycles, so
+    // columns against zero slices would cost as much as any: 1224 instead of 1104
+    // cycles per K step at s = 8, p + q <= 8, BN = 48).  Each block belongs to one of
+    // the issuing warps, dealt by cost: one thread issues a UMMA about every 60-80
+    // cycles at best, more with the drain warps on its scheduler.
+    {
+        p.n_iss = hint.issuers >= 1 && hint.issuers <= kMaxIssuers ? hint.issuers : kMaxIssuers;
+        p.n_iss = std::min(p.n_iss, p.G);
+        std::vector<uint16_t> ops[kMaxGroups];
+        double cost[kMaxGroups] = {0}, load[kMaxIssuers] = {0};
+        int order[kMaxGroups], owner[kMaxGroups];
+        p.mma_per_kstep = 0;
+        for (int g = 0; g < p.G; ++g) {
+            const int lo = p.blk_lo[g], hi = lo + p.blk_nb[g] - 1;
+            order[g] = g;
+            for (int pa = 0; pa < s; ++pa) {
+                const int a = std::max(lo, pa), e = std::min(hi, pa + s - 1);
+                if (a > e) continue;
+                ops[g].push_back(pack_op(pa, a, e - a + 1));
+                cost[g] += std::max(0.5 * (e - a + 1) * p.BN, 32.0 + 0.25 * (e - a + 1) * p.BN);
+            }
+            const auto full = std::find_if(ops[g].begin(), ops[g].end(),
+                                           [&](uint16_t op) { return op_nb(op) == p.blk_nb[g]; });
+            if (full != ops[g].end()) std::swap(*full, ops[g].front());
+            else p.zero_mask |= 1u << g;
+            p.mma_per_kstep += static_cast<int>(ops[g].size());
+        }
+        if (p.mma_per_kstep > kMaxOps) {
+            *err = "too many UMMAs per K step";
+            return false;
+        }
+        std::stable_sort(order, order + p.G, [&](int x, int y) { return cost[x] > cost[y]; });
+        for (int i = 0; i < p.G; ++i) {
+            owner[order[i]] = static_cast<int>(std::min_element(load, load + p.n_iss) - load);
+            load[owner[order[i]]] += cost[order[i]];
+        }
+        for (int i = 0, n = 0; i < p.n_iss; ++i) {
+            for (int g = 0; g < p.G; ++g)
+                if (owner[g] == i)
+                    for (uint16_t op : ops[g]) p.ops[n++] = op;
+            p.op_end[i] = n;
+        }
+    }
     // ---- pipeline: K chunk and stage count (a chunk of 32 bf16 or 64 e4m3 K values
     // is 64 bytes per row and slice)
     const size_t eb = p.f8 ? 1 : 2;
+    const size_t ops_bytes = sizeof(uint32_t) * 4 * p.mma_per_kstep;  // the UMMA lists, decoded
     const size_t budget = kSmemLimit - kSmemReserve;
     const int kc_opts[2] = {p.f8 ? 64 : 32, p.f8 ? 32 : 16};
     const int kmin = kc_opts[1];
     const int force_kc = hint.KC;
     auto stage_of = [&](int kc) {
-        return (static_cast<size_t>(s) * BM * kc + static_cast<size_t>(p.pad_lo + s + p.pad_hi) * p.BN * kc) * eb;
+        return (static_cast<size_t>(s) * BM * kc + static_cast<size_t>(pad_lo + s + pad_hi) * p.BN * kc) * eb;
     };
     p.KC = 0;
     for (int kc : kc_opts) {
@@ -443,51 +512,54 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     p.tiles_n = (N + p.BN - 1) / p.BN;
     p.Mp = p.tiles_m * BM;
     p.Np = p.tiles_n * p.BN;
-    p.b_slice_bytes = static_cast<uint32_t>(p.BN * p.KC * eb);
     p.a_block_bytes = static_cast<uint32_t>(s * BM * p.KC * eb);
-    p.b_block_bytes = static_cast<uint32_t>(s) * p.b_slice_bytes;
-    p.b_region_bytes = static_cast<uint32_t>(p.pad_lo + s + p.pad_hi) * p.b_slice_bytes;
-    p.stage_bytes = p.a_block_bytes + p.b_region_bytes;
+    p.b_block_bytes = static_cast<uint32_t>(s * p.BN * p.KC * eb);
+    p.stage_bytes = p.a_block_bytes + p.b_block_bytes;
     p.a_elems = static_cast<size_t>(p.tiles_m) * p.n_kc * s * BM * p.KC;
     p.b_elems = static_cast<size_t>(p.tiles_n) * p.n_kc * s * p.BN * p.KC;
     p.a_bytes = p.a_elems * eb;
     p.b_bytes = p.b_elems * eb;
-    // ---- double buffering: blocks get a second accumulator range in the TMEM
-    // columns the bins leave free, most frequently drained blocks first (the
-    // order does not depend on K, so problems of one shape class share a plan);
-    // their UMMAs then switch ranges at each drain, and at the end of a tile,
-    // instead of waiting for the drain warps to read the block out.
-    p.dbl_mask = 0;
-    int next_col = J * p.BN;  // buffer 0: bin j at column j BN
-    if (hint.dbl != 0) {
-        int order[kMaxGroups], n = 0;
-        long period[kMaxGroups];  // in K values, not clamped to this K
-        for (int g = 0; g < p.G; ++g) {
-            order[n++] = g;
-            period[g] = 1L << 40;
-            for (int j = p.blk_lo[g]; j < p.blk_lo[g] + p.blk_nb[g]; ++j)
-                period[g] = std::min(period[g], static_cast<long>(std::floor(16777216.0 / (pairs_in_bin(j, s) * v2 * v2))));
-        }
-        std::sort(order, order + n, [&](int x, int y) {
-            return period[x] != period[y] ? period[x] < period[y] : (p.blk_nb[x] != p.blk_nb[y] ? p.blk_nb[x] > p.blk_nb[y] : x < y);
-        });
-        for (int i = 0; i < n; ++i) {
-            const int g = order[i];
-            if (next_col + p.blk_nb[g] * p.BN > 512) continue;
-            p.dbl_mask |= 1u << g;
-            p.blk_col1[g] = next_col;
-            next_col += p.blk_nb[g] * p.BN;
-        }
-    }
-    uint32_t cols = 32;
-    while (cols < static_cast<uint32_t>(next_col)) cols <<= 1;
-    p.tmem_cols = cols;
-    p.smem = static_cast<size_t>(p.stages) * p.stage_bytes + kCtrlBytes;
+    while (p.stages > 1 && p.stages * static_cast<size_t>(p.stage_bytes) + kCtrlBytes + ops_bytes > kSmemLimit) --p.stages;
+    p.smem = static_cast<size_t>(p.stages) * p.stage_bytes + kCtrlBytes + ops_bytes;
     *out = p;
     return true;
 }
 
 }  // namespace
+
+void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, unsigned long long timeout_ns) {
+    std::memset(g, 0, sizeof *g);
+    g->KC = p.KC;
+    g->s = p.cfg.s;
+    g->J = p.cfg.J;
+    g->b = p.cfg.b;
+    g->out_mode = out_mode;
+    g->stages = p.stages;
+    g->stage_bytes = p.stage_bytes;
+    g->a_block_bytes = p.a_block_bytes;
+    g->b_block_bytes = p.b_block_bytes;
+    g->tmem_cols = p.tmem_cols;
+    g->err = err;
+    g->timeout_ns = timeout_ns;
+    g->alpha = 1.0;
+    g->beta = 0.0;
+    g->n_acc = p.n_acc;
+    g->n_iss = p.n_iss;
+    for (int a = 0; a < kMaxAcc; ++a) g->acc_t0[a] = p.acc_t0[a];
+    g->G = p.G;
+    for (int i = 0; i < p.G; ++i) {
+        g->blk_lo[i] = p.blk_lo[i];
+        g->blk_nb[i] = p.blk_nb[i];
+        g->blk_period[i] = p.blk_period[i];
+        g->blk_off[i] = p.blk_off[i];
+        g->blk_first[i] = p.blk_period[i] - p.blk_off[i] % p.blk_period[i];
+        g->blk_col1[i] = p.blk_col1[i];
+    }
+    g->dbl_mask = p.dbl_mask;
+    for (int i = 0; i < p.n_iss; ++i) g->op_end[i] = p.op_end[i];
+    g->zero_mask = p.zero_mask;
+    std::memcpy(g->ops, p.ops, sizeof g->ops);
+}
 
 std::vector<PlanHints> plan_candidates(int M, int N, int K, const OzConfig &cfg, int max_n) {
     std::vector<PlanHints> out;

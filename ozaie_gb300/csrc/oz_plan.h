@@ -25,14 +25,16 @@ struct Plan {
     size_t a_bytes = 0, b_bytes = 0;  // bytes of the slice blocks in HBM
     int n_kc = 0, Kp = 0, Mp = 0, Np = 0, tiles_m = 0, tiles_n = 0;
     int pairs = 0, max_pairs = 0, mma_per_kstep = 0;
-    int pad_lo = 0, pad_hi = 0;
     size_t a_elems = 0, b_elems = 0;  // bf16 elements of the slice blocks in HBM
-    uint32_t a_block_bytes = 0, b_block_bytes = 0, b_slice_bytes = 0, b_region_bytes = 0, stage_bytes = 0;
+    uint32_t a_block_bytes = 0, b_block_bytes = 0, stage_bytes = 0;
     uint32_t tmem_cols = 0;
     size_t smem = 0;
     double model_cycles_per_kstep = 0;  // UMMA cost model of the chosen blocks
-    int blk_lo[kMaxGroups] = {0}, blk_nb[kMaxGroups] = {0}, blk_p0[kMaxGroups] = {0}, blk_p1[kMaxGroups] = {0};
+    int blk_lo[kMaxGroups] = {0}, blk_nb[kMaxGroups] = {0};
     int blk_period[kMaxGroups] = {0}, blk_off[kMaxGroups] = {0};
+    int op_end[kMaxIssuers] = {0};  // the issuers' UMMA lists (GemmArgs)
+    uint32_t zero_mask = 0;
+    uint16_t ops[kMaxOps] = {0};
     int n_acc = 0, acc_t0[kMaxAcc] = {0};  // drain accumulator groups (GemmArgs)
     int n_iss = 1;                         // MMA-issuing warps (1 to 3)
     uint32_t dbl_mask = 0;                 // double-buffered blocks (GemmArgs)
@@ -66,6 +68,10 @@ struct PlanHints {
 // one exists.
 bool make_plan(int M, int N, int K, const OzConfig &cfg, Plan *out, std::string *err, int bin_lo = 0,
                int bin_hi = 1 << 30, const PlanHints *hints = nullptr);
+
+// GEMM launch arguments that follow from the plan alone (shared by all problems
+// of a grouped launch); operands, sizes and tiles are set by the caller.
+void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, unsigned long long timeout_ns);
 
 // Distinct feasible plans for the autotuner (at most max_n), the untuned plan first.
 std::vector<PlanHints> plan_candidates(int M, int N, int K, const OzConfig &cfg, int max_n);

@@ -29,14 +29,17 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
+// The suspend-time hint lets the waiting warp sleep until the phase completes.  A
+// waiting warp that polls instead takes issue slots from the MMA-issuing warp of its
+// scheduler: without the hint the slice-pair GEMM ran 14 % slower (4096^3, s = 8).
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(1000000u)
         : "memory");
     return ok != 0;
 }
@@ -53,6 +56,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const 
         if (*abort) return false;
         if (globaltimer_ns() - t0 > timeout_ns) return false;
     }
+}
+
+// True in one lane of the converged warp, the same one each time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+
+// Barrier `id` of N threads (whole warps).
+template <int ID, int N>
+__device__ __forceinline__ void named_barrier() {
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+
+// Registers per thread of the executing warpgroup.  The shares of all warpgroups must
+// not exceed what the block was launched with, or the increase waits forever.
+template <int R>
+__device__ __forceinline__ void regs_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+template <int R>
+__device__ __forceinline__ void regs_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
 }
 
 // ---------------------------------------------------------- bulk async copy

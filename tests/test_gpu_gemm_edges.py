@@ -1,0 +1,71 @@
+"""The slice-pair GEMM at the edges of its tiles, UMMA lists and conversions, held
+bit for bit to the oracle: sizes one off the tile and the K step, schedules from two
+slices up (a block with more bins than slices has no UMMA that spans it), results that
+cancel to almost nothing, subnormal and overflowing results."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(ozlib, A, B, s, J, hint=None, bits=7):
+    import torch
+    dev = torch.device("cuda", 0)
+    M, K = A.shape
+    N = B.shape[1]
+    dA, dB = torch.from_numpy(np.ascontiguousarray(A)).to(dev), torch.from_numpy(np.ascontiguousarray(B)).to(dev)
+    dC = torch.full((M, N), float("nan"), dtype=torch.float64, device=dev)
+    h = ozlib.Handle()
+    h.set_bits(bits)
+    h.set_slices(s)
+    h.set_bins(J)
+    if hint:
+        h.set_plan_hint(**hint)
+    for _ in range(2):  # the second call finds the first one's buffers
+        rc = h.dgemm_device(M, N, K, dA.data_ptr(), K, dB.data_ptr(), N, dC.data_ptr(), N,
+                            torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, h.last_error()
+        assert h.sync() == 0, h.last_error()
+    cfg = h.config()
+    h.close()
+    return dC.cpu().numpy(), cfg
+
+
+def _same(got, ref, what):
+    bad = np.argwhere(got.view(np.uint64) != ref.view(np.uint64))
+    assert bad.size == 0, (what, bad[:4])
+
+
+@pytest.mark.parametrize("s,J", [(2, 2), (2, 3), (3, 5), (4, 7), (5, 6), (8, 8), (8, 9), (8, 15), (10, 11), (12, 12),
+                                 (16, 16)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (127, 47, 15), (129, 49, 33), (130, 65, 161), (257, 97, 400)])
+def test_edges_bit_exact(ozlib, oracle, s, J, M, N, K):
+    A = oracle.gen_phi((M, K), 71, 1.0)
+    B = oracle.gen_phi((K, N), 72, 1.0)
+    got, cfg = _run(ozlib, A, B, s, J)
+    _same(got, oracle.dgemm(A, B, 7, s, J, 0), cfg)
+
+
+@pytest.mark.parametrize("s,J,blocks", [(2, 3, (3,)), (3, 5, (5,)), (3, 5, (4, 1))])
+def test_block_with_more_bins_than_slices(ozlib, oracle, s, J, blocks):
+    """No UMMA spans such a block: its accumulator is zeroed by the drain instead."""
+    M, N, K = 150, 70, 1100
+    A = oracle.gen_phi((M, K), 73, 1.0)
+    B = oracle.gen_phi((K, N), 74, 1.0)
+    got, cfg = _run(ozlib, A, B, s, J, dict(block_nb=blocks, tile_n=32))
+    assert cfg["block_nb"][:cfg["blocks"]] == list(blocks)
+    _same(got, oracle.dgemm(A, B, 7, s, J, 0), cfg)
+
+
+@pytest.mark.parametrize("s,J", [(8, 8), (8, 15), (11, 12), (16, 16)])
+@pytest.mark.parametrize("scale_a,scale_b", [(1.0, 1.0), (2.0 ** -540, 2.0 ** -530), (2.0 ** 520, 2.0 ** 505)])
+def test_cancelling_and_out_of_range_results(ozlib, oracle, s, J, scale_a, scale_b):
+    """A = [X, X], B = [Y; -Y + D]: most of the sum cancels, so the leading groups of
+    the exact sum are zero or small; scaled results are subnormal or overflow."""
+    M, N, K = 96, 64, 320
+    X, Y = oracle.gen_phi((M, K), 75, 0.5), oracle.gen_phi((K, N), 76, 0.5)
+    D = np.where(np.arange(N) % 3 == 0, 0.0, Y * 2.0 ** -(np.arange(N) % 52))
+    A = np.concatenate([X, X], axis=1) * scale_a
+    B = np.concatenate([Y, -(Y + D)], axis=0) * scale_b
+    got, cfg = _run(ozlib, A, B, s, J)
+    _same(got, oracle.dgemm(A, B, 7, s, J, 0), cfg)
