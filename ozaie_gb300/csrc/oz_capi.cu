@@ -387,6 +387,8 @@ bool ensure_zeroed(DevBuf &buf, bool &dirty, size_t bytes, cudaStream_t st) {
 }
 ozgb_status set_tail_split(ozgb_handle h, const Plan &p, int begin, int end, cudaStream_t st, GemmArgs *g) {
     const TailSplit ts = tail_split_shape(p, g->out_mode, begin, end, sm_count(h->device));
+    // the scratch is zeroed on the stream when it is new: the GEMM then follows a memset
+    if (ts.P > 1 && (h->split_dirty || ts.bytes > h->split.cap)) g->pdl = 0;
     if (ts.P > 1 && !ensure_zeroed(h->split, h->split_dirty, ts.bytes, st))
         return fail(h, OZGB_ERR_ALLOC, "split scratch");
     apply_tail_split(g, ts, begin, end, h->split.p);
@@ -403,9 +405,10 @@ struct HostOut {
     bool copied;  // set when the split path has enqueued every copy of C
 };
 
-// Stages (b) and (c)+(d) for one problem whose exponents are in h->er / h->ec.
+// Stages (b) and (c)+(d) for one problem whose exponents are in h->er / h->ec, or with
+// exponents = true stage (a) too.
 ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, int out_mode, int32_t *raw,
-                               cudaStream_t st, HostOut *ho = nullptr) {
+                               cudaStream_t st, HostOut *ho, bool exponents) {
     if (!h->at.ensure(p.a_bytes) || !h->bt.ensure(p.b_bytes))
         return fail(h, OZGB_ERR_ALLOC, "slice buffers");
     uint16_t *at = static_cast<uint16_t *>(h->at.p), *bt = static_cast<uint16_t *>(h->bt.p);
@@ -413,7 +416,11 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
     // run the separate kernels, whose lighter register and shared-memory use
     // measured faster (4096^3: 0.270 against 0.291 ms)
     const double elems = static_cast<double>(p.Mp + p.Np) * p.n_kc * p.KC;
-    if (elems > 16.0 * 1024 * 1024) {
+    if (exponents) {
+        launch_exp_split(o.A, o.lda, o.ta, o.M, p.Mp, static_cast<int32_t *>(h->er.p), at, o.B, o.ldb, o.tb, o.N, p.Np,
+                         p.BN, static_cast<int32_t *>(h->ec.p), bt, o.K, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.f8, st);
+        h->launches += 1;
+    } else if (elems > 16.0 * 1024 * 1024) {
         launch_split_a(o.A, o.lda, o.M, o.K, static_cast<int32_t *>(h->er.p), p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.Mp, at,
                        st, o.ta, p.f8);
         launch_split_b(o.B, o.ldb, o.K, o.N, static_cast<int32_t *>(h->ec.p), p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.BN,
@@ -450,6 +457,7 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
     g.total_tiles = p.tiles_m * p.tiles_n;
     g.alpha = o.alpha;
     g.beta = o.beta;
+    g.pdl = h->profiling ? 0 : 1;  // the GEMM directly follows the split kernel
     if (out_mode == OUT_PAIRS) {
         // the reference's two sums: bins t < g0 and t >= g0, each modulo 2^64
         g.pair_g0 = reference_first_group(o.K, p.cfg.b, p.cfg.s);
@@ -497,6 +505,7 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
         p.fn(g, t_split, p.smem, st);
         cudaEventRecord(h->ev_part, st);
         if (!pageable && (rc = copy_first())) return rc;
+        g.pdl = 0;
         if ((rc = set_tail_split(h, p, t_split, total, st, &g))) return rc;
         p.fn(g, total - t_split, p.smem, st);
         h->launches += 2;
@@ -530,9 +539,10 @@ ozgb_status enqueue_dgemm(ozgb_handle h, const Operands &o, int mode, cudaStream
     h->last_stream = st;
     if (h->profiling) cudaEventRecord(h->ev[0], st);
     const bool want_ss = h->err_bound > 0.0 && h->opt_slices <= 0;
-    ozgb_status rc = enqueue_exponents(h, o, want_ss, st);
-    if (rc) return rc;
-    if (h->profiling) cudaEventRecord(h->ev[1], st);
+    ozgb_status rc;
+    // the knob's statistics come first: the slice schedule follows from them
+    if (want_ss && (rc = enqueue_exponents(h, o, true, st))) return rc;
+    if (want_ss && h->profiling) cudaEventRecord(h->ev[1], st);
     OzConfig cfg;
     if ((rc = choose_config(h, o, mode, st, &cfg))) return rc;
     // dumps read the slice planes back as bf16
@@ -556,8 +566,16 @@ ozgb_status enqueue_dgemm(ozgb_handle h, const Operands &o, int mode, cudaStream
         return fail(h, OZGB_ERR_UNSUPPORTED, why);
     h->last = p;
     h->have_last = true;
+    const bool fused = !want_ss && one_launch_split(p, o.K);
+    if (fused) {
+        if (!h->er.ensure(sizeof(int32_t) * o.M) || !h->ec.ensure(sizeof(int32_t) * o.N))
+            return fail(h, OZGB_ERR_ALLOC, "exponent buffers");
+    } else if (!want_ss && (rc = enqueue_exponents(h, o, false, st))) {
+        return rc;
+    }
+    if (!want_ss && h->profiling) cudaEventRecord(h->ev[1], st);
     const int om = out_mode_override >= 0 ? out_mode_override : cfg.rounding;
-    if ((rc = enqueue_split_gemm(h, o, p, om, raw, st, ho))) return rc;
+    if ((rc = enqueue_split_gemm(h, o, p, om, raw, st, ho, fused))) return rc;
     if (h->profiling && !(ho && ho->copied)) {
         cudaEventRecord(h->ev[3], st);
         h->ev_recorded = true;

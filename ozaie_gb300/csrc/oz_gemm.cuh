@@ -100,14 +100,21 @@ __device__ __forceinline__ void acc_add_group(long long (*acc)[NA], const uint32
 
 // ------------------------------------------------------------ q -> double
 // The exact sum of an element's accumulator groups, sum_x acc[x] 2^B[x] (B[0] = 0),
-// as a 128-bit window and what lies below it: value = (S + f) 2^low with 0 <= f < 1
-// and sticky = (f != 0).  The bits of a group above the next group's weight are first
-// carried into that group (the groups are at most 37 bits apart and stay below 2^62);
-// then the window takes the groups from the top.  A group that no longer fits (|S| is
-// then past 2^64, well over the 53 bits of a result) only sets sticky.
+// as a 128-bit window S = (hi, lo), two's complement, and what lies below it: value =
+// (S + f) 2^low with 0 <= f < 1 and sticky = (f != 0).  The bits of a group above the
+// next group's weight are first carried into that group (the groups are at most 37
+// bits apart and stay below 2^62); then the window takes the groups from the top.  A
+// group that no longer fits (|S| is then past 2^64, well over the 53 bits of a result)
+// only sets sticky.  64-bit words throughout: the compiler's 128-bit shifts by a
+// variable made this and the rounding 390 instructions, now about 80.
+struct Window {
+    long long hi;
+    unsigned long long lo;
+    bool sticky;
+    int low;
+};
 template <int NA>
-OZ_HD inline void acc_window(const long long (&acc)[NA], int n_acc, const int (&B)[kMaxAcc], __int128 *S_out,
-                             bool *sticky_out, int *low_out) {
+OZ_HD inline Window acc_window(const long long (&acc)[NA], int n_acc, const int (&B)[kMaxAcc]) {
     long long top = acc[0];
     unsigned long long dig[NA];  // dig[x]: group x's bits below group x + 1's weight
 #pragma unroll
@@ -117,27 +124,27 @@ OZ_HD inline void acc_window(const long long (&acc)[NA], int n_acc, const int (&
             dig[x - 1] = static_cast<unsigned long long>(top) & ((1ull << d) - 1ull);
             top = acc[x] + (top >> d);
         }
-    __int128 S = top;
-    bool sticky = false, full = false;
-    int low = B[n_acc - 1];
+    Window w;
+    w.hi = top >> 63;
+    w.lo = static_cast<unsigned long long>(top);
+    w.sticky = false;
+    w.low = B[n_acc - 1];
+    bool full = false;
 #pragma unroll
     for (int x = NA - 1; x >= 1; --x)
         if (x < n_acc) {
             const int d = B[x] - B[x - 1];
-            const long long hi = static_cast<long long>(S >> 64);
             // the first of these fits: |top| < 2^63; else |S| < 2^(126 - d)
-            if (x == n_acc - 1 || (!full && ((hi ^ (hi >> 63)) >> (62 - d)) == 0)) {
-                S = static_cast<__int128>(static_cast<unsigned __int128>(S) << d) +
-                    static_cast<__int128>(dig[x - 1]);
-                low = B[x - 1];
+            if (x == n_acc - 1 || (!full && ((w.hi ^ (w.hi >> 63)) >> (62 - d)) == 0)) {
+                w.hi = static_cast<long long>((static_cast<unsigned long long>(w.hi) << d) | (w.lo >> (64 - d)));
+                w.lo = (w.lo << d) | dig[x - 1];
+                w.low = B[x - 1];
             } else {
                 full = true;
-                sticky = sticky || dig[x - 1] != 0;
+                w.sticky = w.sticky || dig[x - 1] != 0;
             }
         }
-    *S_out = S;
-    *sticky_out = sticky;
-    *low_out = low;
+    return w;
 }
 
 OZ_HD inline int clz64(unsigned long long x) {
@@ -161,17 +168,16 @@ OZ_HD inline unsigned long long round_out_of_range(unsigned long long h, int bia
     return mm;
 }
 
-// Bits of (S + f) 2^e2 as a double: rounded to nearest even (OUT_RN) or the
+// Bits of (S + f) 2^(e2 + low) as a double: rounded to nearest even (OUT_RN) or the
 // reference's truncating decode (OUT_RZ_REF, include/oz_aie.h:129-146: 53 truncated
 // bits and the exponent added modulo 2^64).
-OZ_HD inline unsigned long long window_bits(__int128 S, bool sticky, int e2, int mode) {
-    const bool neg = S < 0;
+OZ_HD inline unsigned long long window_bits(const Window &w, int e2, int mode) {
     // the magnitude's floor: -(S + f) = ~S + (1 - f) when f != 0
-    unsigned __int128 m = static_cast<unsigned __int128>(S);
-    if (neg) m = ~m + (sticky ? 0u : 1u);
-    unsigned long long hi = static_cast<unsigned long long>(m >> 64), lo = static_cast<unsigned long long>(m);
+    const unsigned long long neg = static_cast<unsigned long long>(w.hi >> 63);
+    unsigned long long lo = w.lo ^ neg, hi = static_cast<unsigned long long>(w.hi) ^ neg;
+    if (neg != 0 && !w.sticky) hi += ++lo == 0 ? 1u : 0u;
     if ((hi | lo) == 0) return 0ull;
-    // normalise: the top bit of m to bit 63 of hi, what falls below into its lowest bit
+    // normalise: the top bit to bit 63 of hi, what falls below into its lowest bit
     int L = 128;
     if (hi == 0) {
         hi = lo;
@@ -181,14 +187,15 @@ OZ_HD inline unsigned long long window_bits(__int128 S, bool sticky, int e2, int
     const int n = clz64(hi);
     L -= n;
     hi = (hi << n) | ((lo >> 1) >> (63 - n));
-    if ((lo << n) != 0 || sticky) hi |= 1ull;
-    const unsigned long long sign = neg ? 0x8000000000000000ull : 0ull;
-    const int biased = L + e2 + 1022;
+    if ((lo << n) != 0 || w.sticky) hi |= 1ull;
+    const unsigned long long sign = neg << 63;
+    const int biased = L + e2 + w.low + 1022;
     if (mode == OUT_RZ_REF)
-        return (hi >> 11) - 0x0010000000000000ull + sign + (static_cast<unsigned long long>(static_cast<long long>(biased)) << 52);
+        return (hi >> 11) - 0x0010000000000000ull + sign +
+               (static_cast<unsigned long long>(static_cast<long long>(biased)) << 52);
     if (biased < 1 || biased > 2046) return sign | round_out_of_range(hi, biased);
-    const uint32_t w = static_cast<uint32_t>(hi);
-    const uint32_t up = ((w & 0x7FFu) + 0x3FFu + ((w >> 11) & 1u)) >> 11;
+    const uint32_t w0 = static_cast<uint32_t>(hi);
+    const uint32_t up = ((w0 & 0x7FFu) + 0x3FFu + ((w0 >> 11) & 1u)) >> 11;
     return sign + (static_cast<unsigned long long>(biased - 1) << 52) + (hi >> 11) + up;
 }
 
@@ -343,15 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     const int n_iss = g.n_iss < 1 ? 1 : (g.n_iss > kMaxIssuers ? kMaxIssuers : g.n_iss);  // MMA-issuing warps
     for (int i = threadIdx.x; i < g.op_end[n_iss - 1]; i += kThreads) {
         const uint32_t op = g.ops[i];
-        const int p = op_p(op), lo = op_lo(op), nb = op_nb(op);
-        auto block_of = [&](int bin) {
-            int b = 0;
-            for (int x = 1; x < g.G; ++x) b += bin >= g.blk_lo[x] ? 1 : 0;
-            return b;
-        };
-        const int blk = block_of(lo);
-        int count = 1;  // entries of the block from this one on
-        while (i + count < g.op_end[n_iss - 1] && block_of(op_lo(g.ops[i + count])) == blk) ++count;
+        const int p = op_p(op), lo = op_lo(op), nb = op_nb(op), blk = op_blk(op);
         const uint32_t d0 = static_cast<uint32_t>(lo * BN);
         const uint32_t d1 = ((g.dbl_mask >> blk) & 1u)
                                 ? static_cast<uint32_t>(g.blk_col1[blk] + (lo - g.blk_lo[blk]) * BN)
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         const uint32_t idesc = (F8 ? idesc_e4m3_f32(BM, 16) : idesc_bf16_f32(BM, 16)) & ~(0x3Fu << 17);
         recs[i] = make_uint4(d0 | (d1 << 16),
                              static_cast<uint32_t>(p) * ((BM * KC * 2) >> 4) | (static_cast<uint32_t>(blk) << 16) |
-                                 (static_cast<uint32_t>(count) << 24),
+                                 (static_cast<uint32_t>(op_left(op)) << 24),
                              static_cast<uint32_t>(lo - p) * ((BN * KC * 2) >> 4),
                              idesc | (static_cast<uint32_t>((nb * BN) >> 3) << 17));
     }
@@ -375,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
             }
         }
         mbar_init(mma_done, n_iss);
-        *abort_flag = (*reinterpret_cast<volatile int *>(g.err) != 0) ? 1 : 0;
+        *abort_flag = 0;
         fence_mbar_init();
     }
     if (warp == 1 && lane < g.J) {
@@ -410,6 +409,10 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         __syncthreads();
         tc_fence_after();
     }
+
+    // everything above overlaps the end of the kernel before this one in the stream
+    grid_wait_predecessor();
+    if (threadIdx.x == 0 && *reinterpret_cast<volatile int *>(g.err) != 0) *vabort = 1;
 
     if (warp < kCtrlWarps) {
       regs_dec<kCtrlRegs>();
@@ -707,89 +710,83 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
             }
 
             // --------------------------------------------------- epilogue
+            // A rolled loop over pairs of columns: after each, the accumulators move down by
+            // two registers' worth.  (Unrolled over the columns it is 30 to 40 KB of code that
+            // a small product runs once, from a cold instruction cache: 22000 of the 46000
+            // cycles of a 64^3 product.)
             const int row = tr.mt * BM + 32 * qd + lane;
+            const bool row_ok = row < tr.M;
             const int col0 = tr.nt * BN + part * COLS;
-            if (row < tr.M) {
-                const int er = __ldg(tr.er + row);
-                auto scale_of = [&](int i) { return er + (i < COLS && col0 + i < tr.N ? __ldg(tr.ec + col0 + i) : 0); };
-                const int e_base = -2044 - g.b * (g.J + 1);
-                if (g.out_mode == OUT_PAIRS) {
-                    // the reference's device output: lo, then hi with bits 51..62 = Er + Ec
+            const int er = row_ok ? __ldg(tr.er + row) : 0;
+            const int e_base = er - 2044 - g.b * (g.J + 1);
+            double *crow = tr.c + static_cast<size_t>(row) * tr.ldc;
+            const bool plain = g.alpha == 1.0 && g.beta == 0.0;
+            int B[kMaxAcc];
 #pragma unroll
-                    for (int i = 0; i < COLS; ++i) {
-                        const int col = col0 + i;
-                        if (col < tr.N) {
-                            long long *dst =
-                                reinterpret_cast<long long *>(g.raw) + (static_cast<size_t>(row) * tr.N + col) * 2;
-                            const unsigned long long lo = static_cast<unsigned long long>(acc[i][0]);
-                            unsigned long long hi = 0;
-                            if constexpr (NA > 1) hi = g.n_acc > 1 ? static_cast<unsigned long long>(acc[i][1]) : 0ull;
-                            const unsigned long long scale =
-                                static_cast<unsigned long long>(static_cast<uint32_t>(scale_of(i)));
-                            hi = (hi & 0x8007FFFFFFFFFFFFull) | ((scale & 0xFFFull) << 51);
-                            dst[0] = static_cast<long long>(lo);
-                            dst[1] = static_cast<long long>(hi);
+            for (int x = 0; x < kMaxAcc; ++x) B[x] = g.b * g.acc_t0[x];
+            // the next pair's scale exponents are loaded a step ahead
+            auto col_exp = [&](int col) { return col < tr.N ? __ldg(tr.ec + col) : 0; };
+            int e_next[2] = {col_exp(col0), col_exp(col0 + 1)};
+#pragma unroll 1
+            for (int i = 0; i < COLS; i += 2) {
+                const int col = col0 + i;
+                const int ec[2] = {e_next[0], e_next[1]};
+                if (i + 2 < COLS) {
+                    e_next[0] = col_exp(col + 2);
+                    e_next[1] = col_exp(col + 3);
+                }
+                if (row_ok && col < tr.N) {
+                    const bool two = col + 1 < tr.N;
+                    if (g.out_mode == OUT_PAIRS || g.out_mode == OUT_RAW) {
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            if (u && !two) break;
+                            const size_t at = static_cast<size_t>(row) * tr.N + col + u;
+                            if (g.out_mode == OUT_PAIRS) {
+                                // the reference's device output: lo, then hi with bits 51..62 = Er + Ec
+                                long long *dst = reinterpret_cast<long long *>(g.raw) + at * 2;
+                                unsigned long long hi = 0;
+                                if constexpr (NA > 1)
+                                    hi = g.n_acc > 1 ? static_cast<unsigned long long>(acc[u][1]) : 0ull;
+                                const unsigned long long scale =
+                                    static_cast<unsigned long long>(static_cast<uint32_t>(er + ec[u]));
+                                dst[0] = acc[u][0];
+                                dst[1] = static_cast<long long>((hi & 0x8007FFFFFFFFFFFFull) | ((scale & 0xFFFull) << 51));
+                            } else {
+                                // the exact sum modulo 2^128
+                                unsigned __int128 q = 0;
+#pragma unroll
+                                for (int x = 0; x < NA; ++x)
+                                    if (x < g.n_acc && B[x] < 128)
+                                        q += static_cast<unsigned __int128>(static_cast<__int128>(acc[u][x])) << B[x];
+                                int32_t *dst = g.raw + at * 4;
+#pragma unroll
+                                for (int w = 0; w < 4; ++w) dst[w] = static_cast<int32_t>(q >> (32 * w));
+                            }
                         }
-                    }
-                } else if (g.out_mode == OUT_RAW) {
-#pragma unroll
-                    for (int i = 0; i < COLS; ++i) {
-                        const int col = col0 + i;
-                        if (col < tr.N) {
-                            // the exact sum modulo 2^128
-                            unsigned __int128 q = 0;
-#pragma unroll
-                            for (int x = 0; x < NA; ++x)
-                                if (x < g.n_acc && g.b * g.acc_t0[x] < 128)
-                                    q += static_cast<unsigned __int128>(static_cast<__int128>(acc[i][x]))
-                                         << (g.b * g.acc_t0[x]);
-                            int32_t *dst = g.raw + (static_cast<size_t>(row) * tr.N + col) * 4;
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) dst[w] = static_cast<int32_t>(q >> (32 * w));
-                        }
-                    }
-                } else {
-                    double *crow = tr.c + static_cast<size_t>(row) * tr.ldc;
-                    const bool plain = g.alpha == 1.0 && g.beta == 0.0;
-                    // pairs of columns as one 16-byte store where aligned (fewer, larger
-                    // writes, which matters most when C is host memory)
-                    const bool vec = (reinterpret_cast<uintptr_t>(crow + col0) & 15) == 0;
-                    int B[kMaxAcc];
-#pragma unroll
-                    for (int x = 0; x < kMaxAcc; ++x) B[x] = g.b * g.acc_t0[x];
-                    // the next pair's scale exponents are loaded a step ahead
-                    int es_next[2] = {scale_of(0), scale_of(1)};
-#pragma unroll
-                    for (int i = 0; i < COLS; i += 2) {
-                        const int es[2] = {es_next[0], es_next[1]};
-                        es_next[0] = scale_of(i + 2);
-                        es_next[1] = scale_of(i + 3);
+                    } else {
                         double v[2];
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
-                            const int col = col0 + i + u;
-                            v[u] = 0.0;
-                            if (col < tr.N) {
-                                __int128 S;
-                                bool sticky;
-                                int low;
-                                acc_window<NA>(acc[i + u], g.n_acc, B, &S, &sticky, &low);
-                                v[u] = __longlong_as_double(static_cast<long long>(
-                                    window_bits(S, sticky, es[u] + e_base + low, g.out_mode)));
-                                // BLAS semantics: C is not read when beta == 0
-                                if (!plain)
-                                    v[u] = g.beta == 0.0 ? g.alpha * v[u] : fma(g.beta, crow[col], g.alpha * v[u]);
-                            }
+                            v[u] = __longlong_as_double(static_cast<long long>(
+                                window_bits(acc_window<NA>(acc[u], g.n_acc, B), ec[u] + e_base, g.out_mode)));
+                            // BLAS semantics: C is not read when beta == 0
+                            if (!plain && (u == 0 || two))
+                                v[u] = g.beta == 0.0 ? g.alpha * v[u] : fma(g.beta, crow[col + u], g.alpha * v[u]);
                         }
-                        const int col = col0 + i;
-                        if (vec && col + 1 < tr.N) {
+                        // one 16-byte store where aligned
+                        if (two && (reinterpret_cast<uintptr_t>(crow + col) & 15) == 0) {
                             *reinterpret_cast<double2 *>(crow + col) = make_double2(v[0], v[1]);
                         } else {
-                            if (col < tr.N) crow[col] = v[0];
-                            if (col + 1 < tr.N) crow[col + 1] = v[1];
+                            crow[col] = v[0];
+                            if (two) crow[col + 1] = v[1];
                         }
                     }
                 }
+#pragma unroll
+                for (int k = 0; k + 2 < COLS; ++k)
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) acc[k][a] = acc[k + 2][a];
             }
         }
         if (!ok && !*vabort) {
@@ -845,7 +842,17 @@ void launch_gemm_variant(const GemmArgs &args, int tiles, size_t smem, void *str
     const int range = args.total_tiles - args.tile_begin;
     const int grid = range < device_sm_count() ? range : device_sm_count();
     (void)tiles;
-    kern<<<grid, threads, smem, static_cast<cudaStream_t>(stream)>>>(args);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = args.pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, args);
 }
 
 }  // namespace ozgb

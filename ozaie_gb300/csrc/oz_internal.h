@@ -37,14 +37,20 @@ constexpr int kLaunchRegs = 96, kDrainRegs = 104, kCtrlRegs = 64;
 static_assert(32 * kEpiWarps * kDrainRegs + 32 * kCtrlWarps * kCtrlRegs <= kThreads * kLaunchRegs, "register split");
 constexpr int kMaxIssuers = 3;
 constexpr int kMaxAccWords = 5;
-constexpr int kMaxOps = 512;       // UMMA list of a plan (GemmArgs::ops)
+constexpr int kMaxOps = 384;       // UMMA list of a plan (GemmArgs::ops)
 
 // One entry of a plan's UMMA list: A slice p against the B slices of bins
-// [lo, lo + nb), i.e. q = lo - p .. lo + nb - 1 - p, all within [0, s).
-OZ_HD inline uint16_t pack_op(int p, int lo, int nb) { return static_cast<uint16_t>(p | (lo << 6) | ((nb - 1) << 11)); }
+// [lo, lo + nb) of block blk, i.e. q = lo - p .. lo + nb - 1 - p, all within [0, s);
+// left: entries of the block from this one on.
+OZ_HD inline uint32_t pack_op(int p, int lo, int nb, int blk, int left) {
+    return static_cast<uint32_t>(p) | static_cast<uint32_t>(lo) << 6 | static_cast<uint32_t>(nb - 1) << 11 |
+           static_cast<uint32_t>(blk) << 16 | static_cast<uint32_t>(left) << 20;
+}
 OZ_HD inline int op_p(uint32_t op) { return static_cast<int>(op & 63u); }
 OZ_HD inline int op_lo(uint32_t op) { return static_cast<int>((op >> 6) & 31u); }
 OZ_HD inline int op_nb(uint32_t op) { return static_cast<int>((op >> 11) & 31u) + 1; }
+OZ_HD inline int op_blk(uint32_t op) { return static_cast<int>((op >> 16) & 15u); }
+OZ_HD inline int op_left(uint32_t op) { return static_cast<int>((op >> 20) & 255u); }
 
 // OUT_PAIRS writes the reference's device output (its C buffer before the host
 // decode): per element int64 lo, hi with (Er + Ec) in bits 51..62 of hi.
@@ -109,7 +115,7 @@ struct GemmArgs {
     // store zeros over what they read.
     int op_end[kMaxIssuers];
     uint32_t zero_mask;
-    uint16_t ops[kMaxOps];
+    uint32_t ops[kMaxOps];
     // Double-buffered blocks (bit g of dbl_mask): a second accumulator range at
     // TMEM column blk_col1[g]; after each drain the block's UMMAs switch ranges,
     // so they go on while the drain warps read the other one out.
@@ -141,6 +147,7 @@ struct GemmArgs {
     int n_acc;
     int acc_t0[kMaxAcc];
     int n_iss;  // MMA-issuing warps (1 to 3), each with its own bin blocks
+    int pdl;  // launched as a programmatic dependent of the kernel before it in the stream
     double alpha, beta;  // C = alpha * (A B) + beta * C for OUT_RN / OUT_RZ_REF (1, 0: plain store)
 };
 
@@ -221,6 +228,12 @@ void launch_split_a(const double *A, long lda, int M, int K, const int32_t *er, 
                     int Mp, uint16_t *tiles, void *stream, bool trans = false, bool f8 = false);
 void launch_split_b(const double *B, long ldb, int K, int N, const int32_t *ec, int b, int s, int KC, int n_kc,
                     int BN, int Np, uint16_t *tiles, void *stream, bool trans = false, bool f8 = false);
+// Stages (a) and (b) of both operands in one launch (small operands without the
+// precision knob): exponents of the rows of op(A) and columns of op(B) to er, ec, their
+// slices to at, bt.
+void launch_exp_split(const double *A, long lda, bool ta, int M, int Mp, int32_t *er, uint16_t *at, const double *B,
+                      long ldb, bool tb, int N, int Np, int BN, int32_t *ec, uint16_t *bt, int K, int b, int s, int KC,
+                      int n_kc, bool f8, void *stream);
 int launch_selftest_timeout(int *err, unsigned long long timeout_ns, void *stream);
 // Precision-knob statistics (seven doubles, KnobStats in oz_plan.h) of one
 // problem; zeroes j.out first.

@@ -114,15 +114,23 @@ extern "C" ozgb_status ozgb_dgemm_device_noalloc(int M, int N, int K, const doub
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
     // the previous call's contents stay in the array: zero what is accumulated into
-    if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess ||
-        cudaMemsetAsync(ec, 0, sizeof(int32_t) * N, st) != cudaSuccess) {
+    if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) {
         cudaGetLastError();
         return OZGB_ERR_EXEC;
     }
-    launch_rowmax(dA, lda, M, K, er, nullptr, st);
-    launch_colmax(dB, ldb, K, N, ec, nullptr, st);
-    launch_split_a(dA, lda, M, K, er, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.Mp, at, st, false, p.f8);
-    launch_split_b(dB, ldb, K, N, ec, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.BN, p.Np, bt, st, false, p.f8);
+    if (one_launch_split(p, K)) {
+        launch_exp_split(dA, lda, false, M, p.Mp, er, at, dB, ldb, false, N, p.Np, p.BN, ec, bt, K, p.cfg.b, p.cfg.s,
+                         p.KC, p.n_kc, p.f8, st);
+    } else {
+        if (cudaMemsetAsync(ec, 0, sizeof(int32_t) * N, st) != cudaSuccess) {
+            cudaGetLastError();
+            return OZGB_ERR_EXEC;
+        }
+        launch_rowmax(dA, lda, M, K, er, nullptr, st);
+        launch_colmax(dB, ldb, K, N, ec, nullptr, st);
+        launch_split_a(dA, lda, M, K, er, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.Mp, at, st, false, p.f8);
+        launch_split_b(dB, ldb, K, N, ec, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.BN, p.Np, bt, st, false, p.f8);
+    }
     if (cudaGetLastError() != cudaSuccess) return OZGB_ERR_EXEC;  // a stage (a) or (b) launch
 
     GemmArgs g;
@@ -139,6 +147,7 @@ extern "C" ozgb_status ozgb_dgemm_device_noalloc(int M, int N, int K, const doub
     g.tiles_m = p.tiles_m;
     g.tiles_n = p.tiles_n;
     g.total_tiles = p.tiles_m * p.tiles_n;
+    g.pdl = 1;  // directly after the split kernel
     p.fn(g, p.tiles_m * p.tiles_n, p.smem, st);
     if (cudaGetLastError() != cudaSuccess) return OZGB_ERR_EXEC;  // the slice-pair GEMM launch
     return OZGB_OK;

@@ -406,7 +406,7 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     {
         p.n_iss = hint.issuers >= 1 && hint.issuers <= kMaxIssuers ? hint.issuers : kMaxIssuers;
         p.n_iss = std::min(p.n_iss, p.G);
-        std::vector<uint16_t> ops[kMaxGroups];
+        std::vector<uint32_t> ops[kMaxGroups];
         double cost[kMaxGroups] = {0}, load[kMaxIssuers] = {0};
         int order[kMaxGroups], owner[kMaxGroups];
         p.mma_per_kstep = 0;
@@ -416,11 +416,11 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
             for (int pa = 0; pa < s; ++pa) {
                 const int a = std::max(lo, pa), e = std::min(hi, pa + s - 1);
                 if (a > e) continue;
-                ops[g].push_back(pack_op(pa, a, e - a + 1));
+                ops[g].push_back(pack_op(pa, a, e - a + 1, g, 0));
                 cost[g] += std::max(0.5 * (e - a + 1) * p.BN, 32.0 + 0.25 * (e - a + 1) * p.BN);
             }
             const auto full = std::find_if(ops[g].begin(), ops[g].end(),
-                                           [&](uint16_t op) { return op_nb(op) == p.blk_nb[g]; });
+                                           [&](uint32_t op) { return op_nb(op) == p.blk_nb[g]; });
             if (full != ops[g].end()) std::swap(*full, ops[g].front());
             else p.zero_mask |= 1u << g;
             p.mma_per_kstep += static_cast<int>(ops[g].size());
@@ -437,7 +437,9 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
         for (int i = 0, n = 0; i < p.n_iss; ++i) {
             for (int g = 0; g < p.G; ++g)
                 if (owner[g] == i)
-                    for (uint16_t op : ops[g]) p.ops[n++] = op;
+                    for (size_t k = 0; k < ops[g].size(); ++k)
+                        p.ops[n++] = pack_op(op_p(ops[g][k]), op_lo(ops[g][k]), op_nb(ops[g][k]), g,
+                                             static_cast<int>(ops[g].size() - k));
             p.op_end[i] = n;
         }
     }
@@ -559,6 +561,19 @@ void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, uns
     for (int i = 0; i < p.n_iss; ++i) g->op_end[i] = p.op_end[i];
     g->zero_mask = p.zero_mask;
     std::memcpy(g->ops, p.ops, sizeof g->ops);
+}
+
+bool one_launch_split(const Plan &p, int K) {
+    // A block walks all of K, so K has to be short or the blocks many; the two-window
+    // and e4m3 splits do about twice the work per value.  Measured, one launch against
+    // two, us per call: 64^3 22.7 / 33.0, 512^3 39.1 / 49.4, 1024^3 90.3 / 96.4, 2048^3
+    // 483 / 494, 256 x 256 x 512 37.1 / 45.6, but 256 x 256 x 2048 (48 blocks) 55.7 / 51.4,
+    // 512 x 512 x 4096 148 / 120 and 3000^3 1384 / 1370; e4m3 slices of b = 3: 64^3 26.9 /
+    // 39.9, 2048 x 256 x 1024 279 / 284, 256 x 256 x 2048 141 / 96.
+    const int avoid = 1 + (p.cfg.b == 3 ? 3 : 0);
+    const bool two = p.f8 || p.cfg.s * p.cfg.b > 64 - avoid - ((64 - avoid) % p.cfg.b);
+    const int blocks = p.Mp / 8 + p.Np / 16;
+    return two ? K <= std::max(256, 4 * blocks) : K <= std::min(2048, std::max(1024, 8 * blocks));
 }
 
 std::vector<PlanHints> plan_candidates(int M, int N, int K, const OzConfig &cfg, int max_n) {

@@ -34,7 +34,7 @@ struct Plan {
     int blk_period[kMaxGroups] = {0}, blk_off[kMaxGroups] = {0};
     int op_end[kMaxIssuers] = {0};  // the issuers' UMMA lists (GemmArgs)
     uint32_t zero_mask = 0;
-    uint16_t ops[kMaxOps] = {0};
+    uint32_t ops[kMaxOps] = {0};
     int n_acc = 0, acc_t0[kMaxAcc] = {0};  // drain accumulator groups (GemmArgs)
     int n_iss = 1;                         // MMA-issuing warps (1 to 3)
     uint32_t dbl_mask = 0;                 // double-buffered blocks (GemmArgs)
@@ -72,6 +72,11 @@ bool make_plan(int M, int N, int K, const OzConfig &cfg, Plan *out, std::string 
 // GEMM launch arguments that follow from the plan alone (shared by all problems
 // of a grouped launch); operands, sizes and tiles are set by the caller.
 void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, unsigned long long timeout_ns);
+
+// Whether stages (a) and (b) of a product without the precision knob run as one launch
+// (launch_exp_split), which reads each operand twice with one block per 8 or 16 rows
+// or columns, or as two launches that also spread K over blocks.
+bool one_launch_split(const Plan &p, int K);
 
 // Distinct feasible plans for the autotuner (at most max_n), the untuned plan first.
 std::vector<PlanHints> plan_candidates(int M, int N, int K, const OzConfig &cfg, int max_n);

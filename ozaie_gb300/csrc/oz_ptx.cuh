@@ -58,6 +58,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const 
     }
 }
 
+// Programmatic dependent launch: a kernel launched with the attribute may start while
+// its predecessor in the stream still runs, once all of the predecessor's blocks have
+// passed grid_launch_dependents (or ended); grid_wait_predecessor returns when the
+// predecessor has completed and its writes are visible (at once without the attribute).
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // True in one lane of the converged warp, the same one each time.
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;

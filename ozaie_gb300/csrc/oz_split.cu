@@ -211,6 +211,69 @@ __host__ __device__ inline bool split_two_windows(int b, int s) {
     return s * b > nv0;
 }
 
+// Slices of 8 consecutive K values x of one unit (row of A or column of B) with
+// exponent E: one 16-byte piece per bf16 slice (8 bytes per e4m3 slice) at dst + p
+// slice_elems.  one_window: !split_two_windows(B, s).
+template <int B, bool F8>
+__device__ __forceinline__ void emit8(const double (&x)[8], int E, bool one_window, int s, size_t slice_elems,
+                                      uint8_t *__restrict__ dst) {
+    if (!F8 && one_window) {
+        FastElem fe[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fe[i] = fast_elem(x[i], E);
+#pragma unroll
+        for (int p = 0; p < 64 / B; ++p)
+            if (p < s) *reinterpret_cast<uint4 *>(dst + p * slice_elems * 2) = fast_slice8<B>(fe, p);
+        return;
+    }
+    uint32_t w[8][5], sg[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) split_words(split_value(x[i], E, !one_window), w[i], sg[i]);
+#pragma unroll
+    for (int p = 0; p < 128 / B; ++p) {
+        if (p < s) {
+            if constexpr (F8) {
+                uint2 v;
+                v.x = slices_e4m3x4<B>(w, sg, p);
+                v.y = slices_e4m3x4<B>(w + 4, sg + 4, p);
+                *reinterpret_cast<uint2 *>(dst + p * slice_elems) = v;
+            } else {
+                uint4 v;
+                v.x = slice_bits<B>(w[0], sg[0], p) | (slice_bits<B>(w[1], sg[1], p) << 16);
+                v.y = slice_bits<B>(w[2], sg[2], p) | (slice_bits<B>(w[3], sg[3], p) << 16);
+                v.z = slice_bits<B>(w[4], sg[4], p) | (slice_bits<B>(w[5], sg[5], p) << 16);
+                v.w = slice_bits<B>(w[6], sg[6], p) | (slice_bits<B>(w[7], sg[7], p) << 16);
+                *reinterpret_cast<uint4 *>(dst + p * slice_elems * 2) = v;
+            }
+        }
+    }
+}
+
+// Where the slices of unit u at K values k0 .. k0 + 7 go: blocks [u / TB][k0 / KC][p][TB x KC].
+template <bool F8>
+__device__ __forceinline__ uint8_t *slice_dst(uint16_t *tiles, int u, int k0, int TB, int KC, int n_kc, int s) {
+    const int t = u / TB, r = u % TB, c = k0 / KC, kk = k0 % KC;
+    const size_t at = (static_cast<size_t>(t) * n_kc + c) * s * (static_cast<size_t>(TB) * KC);
+    return reinterpret_cast<uint8_t *>(tiles) +
+           (F8 ? at + canon_offset8(r, kk, KC) : 2 * (at + canon_offset(r, kk, KC)));
+}
+
+// 8 consecutive doubles of a row, 0 from position n on; 128-bit loads where all are in
+// range and aligned.
+__device__ __forceinline__ void load8(const double *__restrict__ src, int n, double (&x)[8]) {
+    if (n >= 8 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double2 d = __ldg(reinterpret_cast<const double2 *>(src) + i);
+            x[2 * i] = d.x;
+            x[2 * i + 1] = d.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = i < n ? __ldg(src + i) : 0.0;
+    }
+}
+
 // A [M][K] row-major -> A slice blocks [mt][c][p][128 x KC].  One thread takes 8
 // consecutive K values of one row and writes one 16-byte piece per slice; a warp
 // covers 8 rows x 32 K (4 core matrices of each slice, 512 contiguous bytes).
@@ -224,75 +287,16 @@ __device__ __forceinline__ void split_a_body(const double *__restrict__ A, long 
     const int k0 = (bx * 32 + kgl) * 8;
     const int Kp = n_kc * KC;
     if (m >= Mp || k0 >= Kp) return;
-    const bool two = split_two_windows(B, s);
-    const int E = m < M ? er[m] : 0;
-    const double *row = A + static_cast<size_t>(m) * lda;
-    if (!F8 && !two) {
-        // one window: 128-bit loads where the row's 8 values are in range and
-        // aligned, the shift-and-add slice conversion
-        double xv[8];
-        const double *src = row + k0;
-        if (!trans && m < M && k0 + 8 <= K && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    double x[8];
+    if (!trans) {
+        load8(A + static_cast<size_t>(m) * lda + k0, m < M ? K - k0 : 0, x);
+    } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const double2 d = __ldg(reinterpret_cast<const double2 *>(src) + i);
-                xv[2 * i] = d.x;
-                xv[2 * i + 1] = d.y;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int k = k0 + i;
-                xv[i] = (m < M && k < K) ? __ldg(trans ? A + static_cast<size_t>(k) * lda + m : row + k) : 0.0;
-            }
-        }
-        FastElem fe[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) fe[i] = fast_elem(xv[i], E);
-        const int mt = m >> 7, r = m & 127, c = k0 / KC, kk = k0 % KC;
-        const size_t slice_elems = static_cast<size_t>(BM) * KC;
-        uint16_t *dst = tiles + (static_cast<size_t>(mt) * n_kc + c) * s * slice_elems + canon_offset(r, kk, KC);
-#pragma unroll
-        for (int p = 0; p < 64 / B; ++p)
-            if (p < s) *reinterpret_cast<uint4 *>(dst + p * slice_elems) = fast_slice8<B>(fe, p);
-        return;
+        for (int i = 0; i < 8; ++i)
+            x[i] = (m < M && k0 + i < K) ? __ldg(A + static_cast<size_t>(k0 + i) * lda + m) : 0.0;
     }
-    uint32_t w[8][5], sg[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int k = k0 + i;
-        const double x = (m < M && k < K) ? __ldg(trans ? A + static_cast<size_t>(k) * lda + m : row + k) : 0.0;
-        split_words(split_value(x, E, two), w[i], sg[i]);
-    }
-    const int mt = m >> 7, r = m & 127, c = k0 / KC, kk = k0 % KC;
-    const size_t slice_elems = static_cast<size_t>(BM) * KC;
-    if constexpr (F8) {
-        // one-byte slices: 8 bytes per thread and slice
-        uint8_t *dst8 = reinterpret_cast<uint8_t *>(tiles) + (static_cast<size_t>(mt) * n_kc + c) * s * slice_elems +
-                        canon_offset8(r, kk, KC);
-#pragma unroll
-        for (int p = 0; p < 128 / B; ++p) {
-            if (p < s) {
-                uint2 v;
-                v.x = slices_e4m3x4<B>(w, sg, p);
-                v.y = slices_e4m3x4<B>(w + 4, sg + 4, p);
-                *reinterpret_cast<uint2 *>(dst8 + p * slice_elems) = v;
-            }
-        }
-        return;
-    }
-    uint16_t *dst = tiles + (static_cast<size_t>(mt) * n_kc + c) * s * slice_elems + canon_offset(r, kk, KC);
-#pragma unroll
-    for (int p = 0; p < 128 / B; ++p) {
-        if (p < s) {
-            uint4 v;
-            v.x = slice_bits<B>(w[0], sg[0], p) | (slice_bits<B>(w[1], sg[1], p) << 16);
-            v.y = slice_bits<B>(w[2], sg[2], p) | (slice_bits<B>(w[3], sg[3], p) << 16);
-            v.z = slice_bits<B>(w[4], sg[4], p) | (slice_bits<B>(w[5], sg[5], p) << 16);
-            v.w = slice_bits<B>(w[6], sg[6], p) | (slice_bits<B>(w[7], sg[7], p) << 16);
-            *reinterpret_cast<uint4 *>(dst + p * slice_elems) = v;
-        }
-    }
+    emit8<B, F8>(x, m < M ? er[m] : 0, !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
+                 slice_dst<F8>(tiles, m, k0, BM, KC, n_kc, s));
 }
 template <int B, bool F8>
 __global__ void k_split_a(const double *__restrict__ A, long lda, int M, int K, const int32_t *__restrict__ er,
@@ -311,69 +315,99 @@ __device__ __forceinline__ void split_b_body(const double *__restrict__ Bm, long
     const int k0 = (by * 8 + (threadIdx.x >> 5)) * 8;
     const int Kp = n_kc * KC;
     if (n >= Np || k0 >= Kp) return;
-    const bool two = split_two_windows(B, s);
-    const int E = n < N ? ec[n] : 0;
-    if (!F8 && !two) {
-        // one window: the shift-and-add slice conversion
-        FastElem fe[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int k = k0 + i;
-            const double x = (n < N && k < K) ? __ldg(trans ? Bm + static_cast<size_t>(n) * ldb + k
-                                                            : Bm + static_cast<size_t>(k) * ldb + n)
-                                              : 0.0;
-            fe[i] = fast_elem(x, E);
-        }
-        const int nt = n / BN, r = n % BN, c = k0 / KC, kk = k0 % KC;
-        const size_t slice_elems = static_cast<size_t>(BN) * KC;
-        uint16_t *dst = tiles + (static_cast<size_t>(nt) * n_kc + c) * s * slice_elems + canon_offset(r, kk, KC);
-#pragma unroll
-        for (int q = 0; q < 64 / B; ++q)
-            if (q < s) *reinterpret_cast<uint4 *>(dst + q * slice_elems) = fast_slice8<B>(fe, q);
-        return;
-    }
-    uint32_t w[8][5], sg[8];
+    double x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int k = k0 + i;
-        const double x =
-            (n < N && k < K) ? __ldg(trans ? Bm + static_cast<size_t>(n) * ldb + k : Bm + static_cast<size_t>(k) * ldb + n)
-                             : 0.0;
-        split_words(split_value(x, E, two), w[i], sg[i]);
+        x[i] = (n < N && k < K) ? __ldg(trans ? Bm + static_cast<size_t>(n) * ldb + k : Bm + static_cast<size_t>(k) * ldb + n)
+                                : 0.0;
     }
-    const int nt = n / BN, r = n % BN, c = k0 / KC, kk = k0 % KC;
-    const size_t slice_elems = static_cast<size_t>(BN) * KC;
-    if constexpr (F8) {
-        uint8_t *dst8 = reinterpret_cast<uint8_t *>(tiles) + (static_cast<size_t>(nt) * n_kc + c) * s * slice_elems +
-                        canon_offset8(r, kk, KC);
-#pragma unroll
-        for (int q = 0; q < 128 / B; ++q) {
-            if (q < s) {
-                uint2 v;
-                v.x = slices_e4m3x4<B>(w, sg, q);
-                v.y = slices_e4m3x4<B>(w + 4, sg + 4, q);
-                *reinterpret_cast<uint2 *>(dst8 + q * slice_elems) = v;
-            }
-        }
-        return;
-    }
-    uint16_t *dst = tiles + (static_cast<size_t>(nt) * n_kc + c) * s * slice_elems + canon_offset(r, kk, KC);
-#pragma unroll
-    for (int q = 0; q < 128 / B; ++q) {
-        if (q < s) {
-            uint4 v;
-            v.x = slice_bits<B>(w[0], sg[0], q) | (slice_bits<B>(w[1], sg[1], q) << 16);
-            v.y = slice_bits<B>(w[2], sg[2], q) | (slice_bits<B>(w[3], sg[3], q) << 16);
-            v.z = slice_bits<B>(w[4], sg[4], q) | (slice_bits<B>(w[5], sg[5], q) << 16);
-            v.w = slice_bits<B>(w[6], sg[6], q) | (slice_bits<B>(w[7], sg[7], q) << 16);
-            *reinterpret_cast<uint4 *>(dst + q * slice_elems) = v;
-        }
-    }
+    emit8<B, F8>(x, n < N ? ec[n] : 0, !split_two_windows(B, s), s, static_cast<size_t>(BN) * KC,
+                 slice_dst<F8>(tiles, n, k0, BN, KC, n_kc, s));
 }
 template <int B, bool F8>
 __global__ void k_split_b(const double *__restrict__ Bm, long ldb, int K, int N, const int32_t *__restrict__ ec,
                           int s, int KC, int n_kc, int BN, int Np, uint16_t *__restrict__ tiles, int trans) {
+    grid_launch_dependents();
     split_b_body<B, F8>(Bm, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, blockIdx.x, blockIdx.y, trans != 0);
+}
+
+// ------------------------------------------- stages (a) and (b) in one launch
+// For small operands without the precision knob: a block takes all of K of a few
+// units, finds their exponents and splits them in a second pass over the same data
+// (from L1 / L2).  One launch and no exponents to zero, instead of a memset and two
+// launches.  Units that are rows of the stored operand (contiguous in K): 8 per block,
+// a warp each for the exponent; columns of it: 16 per block, 128 contiguous bytes of a
+// row per load.
+struct ExpSplitJob {
+    const double *X;
+    long ld;
+    int units, padded, K;  // padded: units rounded up to whole tiles
+    int TB;                // units per tile
+    int rows;              // units are rows of X (1) or columns (0)
+    int32_t *e_out;
+    uint16_t *tiles;
+};
+template <int B, bool F8>
+__device__ __forceinline__ void exp_split_body(const ExpSplitJob &j, int s, int KC, int n_kc, int bx) {
+    const int Kp = n_kc * KC;
+    const bool one = !split_two_windows(B, s);
+    const size_t slice_elems = static_cast<size_t>(j.TB) * KC;
+    if (j.rows) {
+        __shared__ int sh_e[8];
+        const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int uw = bx * 8 + wid;
+        int e = 0;
+        if (uw < j.units) {
+            const double *row = j.X + static_cast<size_t>(uw) * j.ld;
+#pragma unroll 8
+            for (int k = lane; k < j.K; k += 32) e = max(e, exp_field(__ldg(row + k)));
+        }
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) {
+            sh_e[wid] = e;
+            if (uw < j.units) j.e_out[uw] = e;
+        }
+        __syncthreads();
+        const int r8 = threadIdx.x & 7, u = bx * 8 + r8;
+        const int E = sh_e[r8];
+        for (int k0 = (threadIdx.x >> 3) * 8; k0 < Kp; k0 += 256) {
+            double x[8];
+            load8(j.X + static_cast<size_t>(u) * j.ld + k0, u < j.units ? j.K - k0 : 0, x);
+            emit8<B, F8>(x, E, one, s, slice_elems, slice_dst<F8>(j.tiles, u, k0, j.TB, KC, n_kc, s));
+        }
+    } else {
+        __shared__ int sh_c[16][17];
+        const int c = threadIdx.x & 15, kl = threadIdx.x >> 4;
+        const int u = bx * 16 + c;
+        int e = 0;
+        if (u < j.units) {
+#pragma unroll 8
+            for (int k = kl; k < j.K; k += 16) e = max(e, exp_field(__ldg(j.X + static_cast<size_t>(k) * j.ld + u)));
+        }
+        sh_c[kl][c] = e;
+        __syncthreads();
+        int E = 0;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) E = max(E, sh_c[r][c]);
+        if (kl == 0 && u < j.units) j.e_out[u] = E;
+        for (int k0 = kl * 8; k0 < Kp; k0 += 128) {
+            double x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                x[i] = (u < j.units && k0 + i < j.K) ? __ldg(j.X + static_cast<size_t>(k0 + i) * j.ld + u) : 0.0;
+            emit8<B, F8>(x, E, one, s, slice_elems, slice_dst<F8>(j.tiles, u, k0, j.TB, KC, n_kc, s));
+        }
+    }
+}
+template <int B, bool F8>
+__global__ void __launch_bounds__(256) k_exp_split(const __grid_constant__ ExpSplitJob a,
+                                                   const __grid_constant__ ExpSplitJob b, int n0, int s, int KC,
+                                                   int n_kc) {
+    grid_launch_dependents();
+    const int bid = blockIdx.x;
+    if (bid < n0) exp_split_body<B, F8>(a, s, KC, n_kc, bid);
+    else exp_split_body<B, F8>(b, s, KC, n_kc, bid - n0);
 }
 
 // b (1..7) as a template argument: the slice positions become constants.
@@ -838,6 +872,7 @@ __global__ void __launch_bounds__(kStageThreads) k_stage_jobs(const StageJob *__
 // Two jobs of one problem (A and B) in one launch: blocks [0, n0) run j0.
 __global__ void __launch_bounds__(kStageThreads) k_stage_pair(const __grid_constant__ StageJob j0,
                                                               const __grid_constant__ StageJob j1, int n0) {
+    grid_launch_dependents();
     const int bid = blockIdx.x;
     if (bid < n0) run_stage_job<true>(j0, bid);
     else run_stage_job<true>(j1, bid - n0);
@@ -952,6 +987,24 @@ void launch_colmax(const double *B, long ldb, int K, int N, int32_t *ec, double 
     const int rows = 64;
     dim3 grid((N + threads - 1) / threads, (K + rows - 1) / rows);
     k_colmax<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(B, ldb, K, N, rows, ec, ss);
+}
+
+void launch_exp_split(const double *A, long lda, bool ta, int M, int Mp, int32_t *er, uint16_t *at, const double *B,
+                      long ldb, bool tb, int N, int Np, int BN, int32_t *ec, uint16_t *bt, int K, int b, int s, int KC,
+                      int n_kc, bool f8, void *stream) {
+    const ExpSplitJob ja{A, lda, M, Mp, K, BM, ta ? 0 : 1, er, at};
+    const ExpSplitJob jb{B, ldb, N, Np, K, BN, tb ? 1 : 0, ec, bt};
+    const int n0 = Mp / (ja.rows ? 8 : 16), n1 = Np / (jb.rows ? 8 : 16);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define OZ_CALL_ES(BB) k_exp_split<BB, false><<<n0 + n1, 256, 0, st>>>(ja, jb, n0, s, KC, n_kc)
+#define OZ_CALL_ES8(BB) k_exp_split<BB, true><<<n0 + n1, 256, 0, st>>>(ja, jb, n0, s, KC, n_kc)
+    if (f8) {
+        OZ_SPLIT_DISPATCH_F8(b, OZ_CALL_ES8)
+    } else {
+        OZ_SPLIT_DISPATCH(b, OZ_CALL_ES)
+    }
+#undef OZ_CALL_ES
+#undef OZ_CALL_ES8
 }
 
 void launch_split_a(const double *A, long lda, int M, int K, const int32_t *er, int b, int s, int KC, int n_kc,

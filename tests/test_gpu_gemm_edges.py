@@ -69,3 +69,36 @@ def test_cancelling_and_out_of_range_results(ozlib, oracle, s, J, scale_a, scale
     B = np.concatenate([Y, -(Y + D)], axis=0) * scale_b
     got, cfg = _run(ozlib, A, B, s, J)
     _same(got, oracle.dgemm(A, B, 7, s, J, 0), cfg)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("b,s,K", [(7, 8, 1000), (7, 8, 1100), (7, 12, 250), (7, 12, 300), (3, 18, 70), (3, 18, 301),
+                                   (4, 9, 255)])
+def test_one_launch_split_matches_two(ozlib, oracle, b, s, K, ta, tb):
+    """Exponents and slices in one launch (short K) and in two: every operand order,
+    padded odd leading dimensions, one and two windows, both carriers."""
+    import torch
+    M, N = 133, 49
+    A, B = oracle.gen_phi((M, K), 77, 1.0), oracle.gen_phi((K, N), 78, 1.0)
+    A[5] = 0.0
+    B[:, 7] = 0.0
+    dev = torch.device("cuda", 0)
+
+    def stored(x, trans):
+        x = np.ascontiguousarray(x.T if trans else x)
+        buf = torch.full((x.shape[0], x.shape[1] + 3), float("nan"), dtype=torch.float64, device=dev)
+        buf[:, :x.shape[1]] = torch.from_numpy(x)
+        return buf
+
+    dA, dB = stored(A, ta), stored(B, tb)
+    dC = torch.full((M, N), float("nan"), dtype=torch.float64, device=dev)
+    h = ozlib.Handle()
+    h.set_bits(b)
+    h.set_slices(s)
+    h.set_bins(s)
+    rc = h.dgemm_ex(ta, tb, M, N, K, 1.0, dA.data_ptr(), dA.shape[1], dB.data_ptr(), dB.shape[1], 0.0, dC.data_ptr(),
+                    N, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, h.last_error()
+    assert h.sync() == 0, h.last_error()
+    h.close()
+    _same(dC.cpu().numpy(), oracle.dgemm(A, B, b, s, s, 0), (b, s, K, ta, tb))
