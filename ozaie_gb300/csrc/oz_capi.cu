@@ -78,6 +78,7 @@ struct ozgb_context {
     // launches by the kernel itself (zeroed here only when (re)allocated or after a
     // device error)
     DevBuf split;
+    DevBuf norm;  // the slices' norms per tile of A, then of B (Plan::norms)
     bool split_dirty = true;
     KnobJob kjob{};  // the last stage-(a) statistics, for the precision knob
     DevBuf gstat, gslice, gtab;  // grouped calls: statistics, slice planes, job/problem tables
@@ -104,6 +105,7 @@ struct ozgb_context {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool ev_recorded = false;
     long long launches = 0;  // kernels this handle has launched
+    int *err_host = nullptr;  // page-locked copy of the device error word
     std::string msg;
 };
 
@@ -146,6 +148,8 @@ ozgb_status ensure_device(ozgb_handle h) {
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return cuda_fail(h, e, "cudaEventCreate");
     if (!h->err.ensure(sizeof(int))) return fail(h, OZGB_ERR_ALLOC, "device error word");
     cudaMemset(h->err.p, 0, sizeof(int));
+    if (!h->err_host && (e = cudaMallocHost(&h->err_host, sizeof(int))) != cudaSuccess)
+        return cuda_fail(h, e, "error word buffer");
     h->device = dev;
     return OZGB_OK;
 }
@@ -416,15 +420,24 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
     // run the separate kernels, whose lighter register and shared-memory use
     // measured faster (4096^3: 0.270 against 0.291 ms)
     const double elems = static_cast<double>(p.Mp + p.Np) * p.n_kc * p.KC;
+    float *na = nullptr, *nb = nullptr;
+    if (p.norms) {
+        const size_t bytes = sizeof(float) * p.cfg.s * (static_cast<size_t>(p.tiles_m) + p.tiles_n);
+        if (!h->norm.ensure(bytes)) return fail(h, OZGB_ERR_ALLOC, "slice norms");
+        cudaMemsetAsync(h->norm.p, 0, bytes, st);
+        na = static_cast<float *>(h->norm.p);
+        nb = na + static_cast<size_t>(p.cfg.s) * p.tiles_m;
+    }
     if (exponents) {
         launch_exp_split(o.A, o.lda, o.ta, o.M, p.Mp, static_cast<int32_t *>(h->er.p), at, o.B, o.ldb, o.tb, o.N, p.Np,
-                         p.BN, static_cast<int32_t *>(h->ec.p), bt, o.K, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.f8, st);
+                         p.BN, static_cast<int32_t *>(h->ec.p), bt, o.K, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.f8, st, na,
+                         nb);
         h->launches += 1;
-    } else if (elems > 16.0 * 1024 * 1024) {
+    } else if (elems > 16.0 * 1024 * 1024 || na) {
         launch_split_a(o.A, o.lda, o.M, o.K, static_cast<int32_t *>(h->er.p), p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.Mp, at,
-                       st, o.ta, p.f8);
+                       st, o.ta, p.f8, na);
         launch_split_b(o.B, o.ldb, o.K, o.N, static_cast<int32_t *>(h->ec.p), p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.BN,
-                       p.Np, bt, st, o.tb, p.f8);
+                       p.Np, bt, st, o.tb, p.f8, nb);
         h->launches += 2;
     } else {
         StageJob ja{}, jb{};
@@ -455,6 +468,8 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
     g.tiles_m = p.tiles_m;
     g.tiles_n = p.tiles_n;
     g.total_tiles = p.tiles_m * p.tiles_n;
+    g.na = na;
+    g.nb = nb;
     g.alpha = o.alpha;
     g.beta = o.beta;
     g.pdl = h->profiling ? 0 : 1;  // the GEMM directly follows the split kernel
@@ -584,11 +599,12 @@ ozgb_status enqueue_dgemm(ozgb_handle h, const Operands &o, int mode, cudaStream
 }
 
 ozgb_status check_device_error(ozgb_handle h, cudaStream_t st) {
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_fail(h, e, "kernel execution");
-    int word = 0;
-    e = cudaMemcpy(&word, h->err.p, sizeof(int), cudaMemcpyDeviceToHost);
+    // the error word follows the work on the stream into page-locked memory: one wait
+    cudaError_t e = cudaMemcpyAsync(h->err_host, h->err.p, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_fail(h, e, "error word readback");
+    e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(h, e, "kernel execution");
+    const int word = *h->err_host;
     if (word != 0) {
         cudaMemset(h->err.p, 0, sizeof(int));
         h->split_dirty = true;  // a stopped kernel may have left split sums behind
@@ -677,7 +693,7 @@ struct GroupLaunch {
 
 // The launch-level fields of a plan's GemmArgs as a fixed array (no allocation):
 // problems with equal arrays share a grouped launch.
-constexpr int kLaunchFields = 16 + kMaxAcc + 5 * kMaxGroups;
+constexpr int kLaunchFields = 16 + kMaxAcc + 4 * kMaxGroups;
 struct LaunchFields {
     long long v[kLaunchFields];
     int n = 0;
@@ -691,7 +707,7 @@ LaunchFields launch_fields(const GemmArgs &g, const Plan &p) {
     for (long long x : head) f.v[f.n++] = x;
     for (int a = 0; a < kMaxAcc; ++a) f.v[f.n++] = g.acc_t0[a];
     for (int i = 0; i < g.G; ++i)
-        for (long long x : {g.blk_lo[i], g.blk_nb[i], g.blk_period[i], g.blk_off[i], g.blk_col1[i]})
+        for (long long x : {g.blk_lo[i], g.blk_nb[i], g.blk_period[i], g.blk_col1[i]})
             f.v[f.n++] = x;
     unsigned long long h = 1469598103934665603ull;  // FNV-1a over the words
     for (int i = 0; i < f.n; ++i) h = (h ^ static_cast<unsigned long long>(f.v[i])) * 1099511628211ull;
@@ -708,7 +724,7 @@ std::vector<long long> launch_key(const GemmArgs &g, const Plan &p) {
 
 // The grouped launches of n problems with the given plans and device addresses
 // of their slice blocks and exponents.
-std::vector<GroupLaunch> build_group_launches(const ozgb_problem *probs, int n, const std::vector<Plan> &plans,
+std::vector<GroupLaunch> build_group_launches(const ozgb_problem *probs, int n, const std::vector<PlanRef> &plans,
                                               const std::vector<const uint8_t *> &a_tiles,
                                               const std::vector<const uint8_t *> &b_tiles,
                                               const std::vector<const int32_t *> &er,
@@ -717,13 +733,13 @@ std::vector<GroupLaunch> build_group_launches(const ozgb_problem *probs, int n, 
     std::vector<int> order(n);
     for (int i = 0; i < n; ++i) order[i] = i;
     auto cost = [&](int i) {
-        return static_cast<double>(plans[i].tiles_m) * plans[i].tiles_n * plans[i].n_kc * plans[i].pairs;
+        return static_cast<double>(plans[i]->tiles_m) * plans[i]->tiles_n * plans[i]->n_kc * plans[i]->pairs;
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
     std::vector<GroupLaunch> out;
     std::vector<LaunchFields> keys;  // of out's launches (few: a linear scan of hashes)
     for (int i : order) {
-        const Plan &p = plans[i];
+        const Plan &p = *plans[i];
         GemmArgs g;
         gemm_args_from_plan(&g, p, p.cfg.rounding, err, timeout_ns);
         const LaunchFields key = launch_fields(g, p);
@@ -886,7 +902,7 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
     ozgb_status rc = run_phase(h, graph, key1, &h->gkey1, &h->gexec1, st, [&](cudaStream_t s) -> ozgb_status {
         // column maxima and sums are accumulated atomically: start from zero
         cudaMemsetAsync(gs, 0, total, s);
-        launch_stage_jobs(dja, dba, static_cast<int>(ja.jobs.size()), ja.total, s);
+        launch_stage_jobs(1, dja, dba, static_cast<int>(ja.jobs.size()), ja.total, s);
         if (n_adapt > 0) {
             launch_knob_grouped(dkj, n_adapt, s);
             cudaMemcpyAsync(h->knob_host, knob_dev, sizeof(KnobStats) * n_adapt, cudaMemcpyDeviceToHost, s);
@@ -913,7 +929,7 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
     }
 
     // ---- plans
-    std::vector<Plan> plans(n);
+    std::vector<PlanRef> plans(n);
     for (int i = 0; i < n; ++i) {
         OzConfig cfg = resolve_config(h, probs[i].K, mode);
         if (s_pick[i].s > 0) {
@@ -922,19 +938,19 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
             cfg.J = s_pick[i].J;
         }
         std::string why;
-        if (!make_plan(probs[i].M, probs[i].N, probs[i].K, cfg, &plans[i], &why))
+        if (!(plans[i] = find_plan(probs[i].M, probs[i].N, probs[i].K, cfg, &why)))
             return fail(h, OZGB_ERR_UNSUPPORTED, "problem " + std::to_string(i) + ": " + why);
-        probs[i].slices_used = plans[i].cfg.s;
-        probs[i].bins_used = plans[i].cfg.J;
+        probs[i].slices_used = plans[i]->cfg.s;
+        probs[i].bins_used = plans[i]->cfg.J;
     }
     // ---- phase 2: stage (b) for every problem (one launch) and the GEMMs
     std::vector<size_t> a_off(n), b_off(n);
     size_t sl_total = 0;
     for (int i = 0; i < n; ++i) {
         a_off[i] = sl_total;
-        sl_total += align256(plans[i].a_bytes);
+        sl_total += align256(plans[i]->a_bytes);
         b_off[i] = sl_total;
-        sl_total += align256(plans[i].b_bytes);
+        sl_total += align256(plans[i]->b_bytes);
     }
     if (!h->gslice.ensure(sl_total)) return fail(h, OZGB_ERR_ALLOC, "grouped slice buffer");
     uint8_t *gsl = static_cast<uint8_t *>(h->gslice.p);
@@ -943,7 +959,7 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
     key2.insert(key2.end(), {reinterpret_cast<long long>(gsl), reinterpret_cast<long long>(h->err.p),
                              static_cast<long long>(h->timeout_ns)});
     for (int i = 0; i < n; ++i) {
-        const Plan &p = plans[i];
+        const Plan &p = *plans[i];
         key2.insert(key2.end(), {reinterpret_cast<long long>(probs[i].C), probs[i].ldc, p.cfg.b, p.cfg.s, p.cfg.J,
                                  p.cfg.rounding, p.BN, p.KC, p.stages, p.G});
     }
@@ -992,7 +1008,7 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
     JobList jb;
     for (int i = 0; i < n; ++i) {
         const ozgb_problem &pb = probs[i];
-        const Plan &p = plans[i];
+        const Plan &p = *plans[i];
         StageJob j{};
         j.kind = JOB_SPLIT_A, j.X = pb.A, j.ld = pb.lda, j.rows = pb.M, j.cols = pb.K;
         j.e_in = reinterpret_cast<int32_t *>(at(so[i].er));
@@ -1019,13 +1035,13 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
     std::vector<int> order(n);
     for (int i = 0; i < n; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-        return static_cast<double>(plans[x].tiles_m) * plans[x].tiles_n * plans[x].n_kc * plans[x].pairs >
-               static_cast<double>(plans[y].tiles_m) * plans[y].tiles_n * plans[y].n_kc * plans[y].pairs;
+        return static_cast<double>(plans[x]->tiles_m) * plans[x]->tiles_n * plans[x]->n_kc * plans[x]->pairs >
+               static_cast<double>(plans[y]->tiles_m) * plans[y]->tiles_n * plans[y]->n_kc * plans[y]->pairs;
     });
     const int n_streams = h->grouped_launch ? static_cast<int>(launches.size()) : n;
     const int n_aux = std::max(1, std::min(n_streams, static_cast<int>(ozgb_context::kAux)));
     rc = run_phase(h, graph, key2, &h->gkey2, &h->gexec2, st, [&](cudaStream_t s) -> ozgb_status {
-        launch_stage_jobs(djb, dbb, static_cast<int>(jb.jobs.size()), jb.total, s);
+        launch_stage_jobs(2, djb, dbb, static_cast<int>(jb.jobs.size()), jb.total, s);
         if (prof) cudaEventRecord(h->ev[2], s);
         cudaEventRecord(h->ev_fork, s);
         for (int a = 0; a < n_aux; ++a) cudaStreamWaitEvent(h->aux[a], h->ev_fork, 0);
@@ -1035,7 +1051,7 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
         }
         for (int r = 0; r < n && !h->grouped_launch; ++r) {
             const int k = order[r];
-            const Plan &p = plans[k];
+            const Plan &p = *plans[k];
             GemmArgs g;
             gemm_args_from_plan(&g, p, p.cfg.rounding, static_cast<int *>(h->err.p), h->timeout_ns);
             g.a_tiles = reinterpret_cast<const uint16_t *>(gsl + a_off[k]);
@@ -1067,7 +1083,7 @@ ozgb_status enqueue_grouped(ozgb_handle h, ozgb_problem *probs, int n, int mode,
         cudaEventRecord(h->ev[3], st);
         h->ev_recorded = true;
     }
-    h->last = plans[n - 1];
+    h->last = *plans[n - 1];
     h->have_last = true;
     return OZGB_OK;
 }
@@ -1103,7 +1119,7 @@ ozgb_status ozgb_release(ozgb_handle h) {
     std::lock_guard<std::mutex> lk(h->mu);
     if (h->device >= 0) cudaSetDevice(h->device);
     for (DevBuf *b : {&h->a, &h->b, &h->c, &h->at, &h->bt, &h->er, &h->ec, &h->raw, &h->knob, &h->kpart, &h->gstat,
-                      &h->gslice, &h->gtab, &h->split})
+                      &h->gslice, &h->gtab, &h->split, &h->norm})
         b->release();
     h->split_dirty = true;
     // captured grouped graphs refer to the released buffers
@@ -1133,6 +1149,7 @@ ozgb_status ozgb_destroy(ozgb_handle h) {
         if (h->ev_part) cudaEventDestroy(h->ev_part);
         if (h->ev_part_copied) cudaEventDestroy(h->ev_part_copied);
         if (h->knob_host) cudaFreeHost(h->knob_host);
+        if (h->err_host) cudaFreeHost(h->err_host);
     }
     delete h;
     return OZGB_OK;
@@ -1636,11 +1653,11 @@ int ozgb_grouped_layout_check(const ozgb_problem *probs, int n, int slices, int 
     cfg.s = slices;
     cfg.J = bins > 0 ? bins : slices;
     cfg.rounding = OUT_RN;
-    std::vector<Plan> plans(n);
+    std::vector<PlanRef> plans(n);
     for (int i = 0; i < n; ++i) {
         std::string why;
         if (probs[i].M < 1 || probs[i].N < 1 || probs[i].K < 1 || probs[i].ldc < probs[i].N) return -2;
-        if (!make_plan(probs[i].M, probs[i].N, probs[i].K, cfg, &plans[i], &why)) return -3;
+        if (!(plans[i] = find_plan(probs[i].M, probs[i].N, probs[i].K, cfg, &why))) return -3;
     }
     // stand-in device addresses laid out as enqueue_grouped lays them out
     const uintptr_t slice_base = uintptr_t(1) << 40, exp_base = uintptr_t(1) << 41;
@@ -1650,9 +1667,9 @@ int ozgb_grouped_layout_check(const ozgb_problem *probs, int n, int slices, int 
     size_t sl = 0, ex = 0;
     for (int i = 0; i < n; ++i) {
         a_lo[i] = slice_base + sl;
-        sl += align256(plans[i].a_bytes);
+        sl += align256(plans[i]->a_bytes);
         b_lo[i] = slice_base + sl;
-        sl += align256(plans[i].b_bytes);
+        sl += align256(plans[i]->b_bytes);
         er_lo[i] = exp_base + ex;
         ex += align256(sizeof(int32_t) * probs[i].M);
         ec_lo[i] = exp_base + ex;
@@ -1669,7 +1686,7 @@ int ozgb_grouped_layout_check(const ozgb_problem *probs, int n, int slices, int 
     std::map<uintptr_t, int> by_a;
     for (int i = 0; i < n; ++i) by_a[a_lo[i]] = i;
     std::vector<std::vector<char>> seen(n);
-    for (int i = 0; i < n; ++i) seen[i].assign(static_cast<size_t>(plans[i].tiles_m) * plans[i].tiles_n, 0);
+    for (int i = 0; i < n; ++i) seen[i].assign(static_cast<size_t>(plans[i]->tiles_m) * plans[i]->tiles_n, 0);
     for (const GroupLaunch &L : launches) {
         const GemmArgs &g = L.g;
         if (g.total_tiles != static_cast<int>(L.tile_prob.size()) || g.split_parts != 1) return -4;
@@ -1683,7 +1700,7 @@ int ozgb_grouped_layout_check(const ozgb_problem *probs, int n, int slices, int 
             const auto found = by_a.find(reinterpret_cast<uintptr_t>(P.a_tiles));
             if (found == by_a.end()) return -6;
             const int i = found->second;
-            const Plan &p = plans[i];
+            const Plan &p = *plans[i];
             if (p.fn != L.plan->fn || p.a_block_bytes != g.a_block_bytes || p.b_block_bytes != g.b_block_bytes ||
                 p.stage_bytes != g.stage_bytes || p.n_kc != tr.n_kc)
                 return -7;

@@ -37,6 +37,7 @@ constexpr int kLaunchRegs = 96, kDrainRegs = 104, kCtrlRegs = 64;
 static_assert(32 * kEpiWarps * kDrainRegs + 32 * kCtrlWarps * kCtrlRegs <= kThreads * kLaunchRegs, "register split");
 constexpr int kMaxIssuers = 3;
 constexpr int kMaxAccWords = 5;
+constexpr int kMaxNormSlices = 16; // slices of products whose drains follow the data (Plan::norms)
 constexpr int kMaxOps = 384;       // UMMA list of a plan (GemmArgs::ops)
 
 // One entry of a plan's UMMA list: A slice p against the B slices of bins
@@ -102,13 +103,17 @@ struct GemmArgs {
     uint32_t tmem_cols;
     int *err;
     unsigned long long timeout_ns;
-    // Bin blocks, the drain groups.  Block g holds bins [lo, lo + nb) and is
-    // drained after chunk c when (c + 1 + off) % period == 0, and after the last
-    // chunk.
+    // Bin blocks, the drain groups.  Block g holds bins [lo, lo + nb) and is drained
+    // every blk_period chunks at most, staggered (DrainSchedule), and after the last chunk.
     int G;
     int blk_lo[kMaxGroups], blk_nb[kMaxGroups];
-    int blk_period[kMaxGroups], blk_off[kMaxGroups];
-    int blk_first[kMaxGroups];  // chunks up to and including its first drain
+    int blk_period[kMaxGroups];
+    // Data-dependent drains (null: none): na[mt s + p] is the largest, over the rows of
+    // tile mt and the K chunks, sum of squares of slice p's digits in the chunk; nb[nt s +
+    // q] likewise for the columns.  By Cauchy-Schwarz a chunk adds at most
+    // sum_{p+q=j} sqrt(na[p] nb[q]) to bin j, in every order of its terms, so a block may
+    // go as many chunks between drains as keep that below 2^24 (at least blk_period).
+    const float *na, *nb;
     // UMMAs of a K step (pack_op): issuer i's are ops[op_end[i - 1], op_end[i]), those
     // of a block together, first one that spans the block.  Blocks of zero_mask have no
     // such UMMA (more bins than slices): theirs all accumulate, and the drain warps
@@ -225,24 +230,26 @@ void launch_colmax(const double *B, long ldb, int K, int N, int32_t *ec, double 
 // trans: A is stored K x M (element (m, k) at A[k * lda + m]); B is stored N x K.
 // f8: one-byte e4m3 slices (b <= 4), in the byte layout of a bf16 block of half the K chunk.
 void launch_split_a(const double *A, long lda, int M, int K, const int32_t *er, int b, int s, int KC, int n_kc,
-                    int Mp, uint16_t *tiles, void *stream, bool trans = false, bool f8 = false);
+                    int Mp, uint16_t *tiles, void *stream, bool trans = false, bool f8 = false, float *norm = nullptr);
 void launch_split_b(const double *B, long ldb, int K, int N, const int32_t *ec, int b, int s, int KC, int n_kc,
-                    int BN, int Np, uint16_t *tiles, void *stream, bool trans = false, bool f8 = false);
+                    int BN, int Np, uint16_t *tiles, void *stream, bool trans = false, bool f8 = false, float *norm = nullptr);
+// norm, norm_a, norm_b: the tiles' norms (GemmArgs::na, nb; zeroed before; b = 7, bf16, at most
+// kMaxNormSlices slices), null when not wanted.
 // Stages (a) and (b) of both operands in one launch (small operands without the
 // precision knob): exponents of the rows of op(A) and columns of op(B) to er, ec, their
 // slices to at, bt.
 void launch_exp_split(const double *A, long lda, bool ta, int M, int Mp, int32_t *er, uint16_t *at, const double *B,
                       long ldb, bool tb, int N, int Np, int BN, int32_t *ec, uint16_t *bt, int K, int b, int s, int KC,
-                      int n_kc, bool f8, void *stream);
+                      int n_kc, bool f8, void *stream, float *norm_a = nullptr, float *norm_b = nullptr);
 int launch_selftest_timeout(int *err, unsigned long long timeout_ns, void *stream);
 // Precision-knob statistics (seven doubles, KnobStats in oz_plan.h) of one
 // problem; zeroes j.out first.
 void launch_knob_stats(const KnobJob &j, void *stream);
 // Grid sizes of the per-problem stage kernels (blocks in x and y of 256 threads).
 void stage_grid(const StageJob &j, int *gx, int *gy);
-// Grouped launches: all jobs in one grid (block0[i] = first block of job i,
-// block0[n_jobs] = total), and the knob reduction of n problems.
-void launch_stage_jobs(const StageJob *jobs, const int *block0, int n_jobs, int total_blocks, void *stream);
+// Grouped launches: all jobs of stage (a) (stage = 1) or (b) (2) in one grid (block0[i]
+// = first block of job i, block0[n_jobs] = total), and the knob reduction of n problems.
+void launch_stage_jobs(int stage, const StageJob *jobs, const int *block0, int n_jobs, int total_blocks, void *stream);
 // Two jobs (for example the A and B halves of one stage) in one launch; the grid
 // sizes are filled in here.
 void launch_stage_pair(StageJob j0, StageJob j1, void *stream);

@@ -117,13 +117,10 @@ struct PlanKeyHash {
     }
 };
 std::mutex g_plan_mu;
-std::unordered_map<PlanKey, Plan, PlanKeyHash> g_plans;
+std::unordered_map<PlanKey, PlanRef, PlanKeyHash> g_plans;
 }  // namespace
 
-bool make_plan(int M, int N, int K, const OzConfig &cfg, Plan *out, std::string *err, int bin_lo, int bin_hi,
-               const PlanHints *hints) {
-    if (hints)
-        return make_plan_uncached(M, N, K, cfg, out, err, bin_lo, bin_hi, hints);
+PlanRef find_plan(int M, int N, int K, const OzConfig &cfg, std::string *err, int bin_lo, int bin_hi) {
     long gen;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -133,17 +130,23 @@ bool make_plan(int M, int N, int K, const OzConfig &cfg, Plan *out, std::string 
     {
         std::lock_guard<std::mutex> lk(g_plan_mu);
         auto it = g_plans.find(key);
-        if (it != g_plans.end()) {
-            *out = it->second;
-            return true;
-        }
+        if (it != g_plans.end()) return it->second;
     }
-    Plan p;
-    if (!make_plan_uncached(M, N, K, cfg, &p, err, bin_lo, bin_hi, nullptr)) return false;
+    auto p = std::make_shared<Plan>();
+    if (!make_plan_uncached(M, N, K, cfg, p.get(), err, bin_lo, bin_hi, nullptr)) return nullptr;
     std::lock_guard<std::mutex> lk(g_plan_mu);
     if (g_plans.size() > 8192) g_plans.clear();
     g_plans[key] = p;
-    *out = p;
+    return p;
+}
+
+bool make_plan(int M, int N, int K, const OzConfig &cfg, Plan *out, std::string *err, int bin_lo, int bin_hi,
+               const PlanHints *hints) {
+    if (hints)
+        return make_plan_uncached(M, N, K, cfg, out, err, bin_lo, bin_hi, hints);
+    const PlanRef p = find_plan(M, N, K, cfg, err, bin_lo, bin_hi);
+    if (!p) return false;
+    *out = *p;
     return true;
 }
 
@@ -507,11 +510,15 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
         p.blk_period[g] = per;
         p.min_period = std::min(p.min_period, per);
     }
-    // stagger the drains of different blocks across chunks
-    for (int g = 0; g < p.G; ++g) p.blk_off[g] = (g * p.blk_period[g]) / std::max(1, p.G);
-
     p.tiles_m = (M + BM - 1) / BM;
     p.tiles_n = (N + p.BN - 1) / p.BN;
+    // Drains that follow the data (single products): the split then also takes the
+    // digits' norms, about 15 % more work per value, which pays when a tile drains often
+    // by the worst case and the GEMM has more than two tiles per SM.  GEMM at 4096^3, s =
+    // 8: p + q <= 8 3.68 -> 3.29 ms, full set 5.67 -> 5.07; calls at 2048^3 490 -> 476 and 830
+    // -> 775 us, but 1024^3 (128 tiles) 89 -> 95, 512 x 512 x 4096 122 -> 127.
+    p.norms = !p.f8 && b == 7 && s <= kMaxNormSlices && p.n_kc > 2 * p.min_period &&
+              static_cast<long long>(p.tiles_m) * p.tiles_n > 2 * 152;
     p.Mp = p.tiles_m * BM;
     p.Np = p.tiles_n * p.BN;
     p.a_block_bytes = static_cast<uint32_t>(s * BM * p.KC * eb);
@@ -553,8 +560,6 @@ void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, uns
         g->blk_lo[i] = p.blk_lo[i];
         g->blk_nb[i] = p.blk_nb[i];
         g->blk_period[i] = p.blk_period[i];
-        g->blk_off[i] = p.blk_off[i];
-        g->blk_first[i] = p.blk_period[i] - p.blk_off[i] % p.blk_period[i];
         g->blk_col1[i] = p.blk_col1[i];
     }
     g->dbl_mask = p.dbl_mask;
@@ -721,10 +726,10 @@ Schedule choose_schedule(const KnobStats &k, int M, int N, int K, const OzConfig
             OzConfig c = base;
             c.s = s;
             c.J = J;
-            Plan p;
             std::string why;
-            if (!make_plan(M, N, K, c, &p, &why)) break;  // a larger J needs at least as much
-            const double ms = plan_time_model(p, M, N, K, sms);
+            const PlanRef p = find_plan(M, N, K, c, &why);
+            if (!p) break;  // a larger J needs at least as much
+            const double ms = plan_time_model(*p, M, N, K, sms);
             if (!best.s || ms < best.ms * (1.0 - 1e-9)) {
                 best.s = s;
                 best.J = J;

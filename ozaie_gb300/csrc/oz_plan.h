@@ -3,6 +3,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -31,7 +32,8 @@ struct Plan {
     size_t smem = 0;
     double model_cycles_per_kstep = 0;  // UMMA cost model of the chosen blocks
     int blk_lo[kMaxGroups] = {0}, blk_nb[kMaxGroups] = {0};
-    int blk_period[kMaxGroups] = {0}, blk_off[kMaxGroups] = {0};
+    int blk_period[kMaxGroups] = {0};
+    bool norms = false;  // the split takes the slices' norms, and the drains follow them (GemmArgs::na)
     int op_end[kMaxIssuers] = {0};  // the issuers' UMMA lists (GemmArgs)
     uint32_t zero_mask = 0;
     uint32_t ops[kMaxOps] = {0};
@@ -77,6 +79,12 @@ void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, uns
 // (launch_exp_split), which reads each operand twice with one block per 8 or 16 rows
 // or columns, or as two launches that also spread K over blocks.
 bool one_launch_split(const Plan &p, int K);
+
+// The plan without hints, shared with the process-wide cache (null: refused).  Callers
+// that plan many products (the knob's search, grouped calls) keep the reference rather
+// than a copy of the plan and its UMMA lists.
+using PlanRef = std::shared_ptr<const Plan>;
+PlanRef find_plan(int M, int N, int K, const OzConfig &cfg, std::string *err, int bin_lo = 0, int bin_hi = 1 << 30);
 
 // Distinct feasible plans for the autotuner (at most max_n), the untuned plan first.
 std::vector<PlanHints> plan_candidates(int M, int N, int K, const OzConfig &cfg, int max_n);

@@ -121,18 +121,6 @@ __device__ __forceinline__ void split_words(const SplitState &st, uint32_t (&w)[
     sign = st.neg ? 0x8000u : 0u;
 }
 
-// bf16 bits of slice p (b = B bits at bit position B*p from the top), signed:
-// the magnitude v < 2^8 becomes a float through the FP32 adder (2^23 + v - 2^23,
-// exact) rather than the slower integer conversion; +0 for zero slices.
-template <int B>
-__device__ __forceinline__ uint32_t slice_bits(const uint32_t (&w)[5], uint32_t sign, int p) {
-    const int pos = B * p;
-    const int idx = pos >> 5, off = pos & 31;
-    const uint32_t v = __funnelshift_l(w[idx + 1], w[idx], off) >> (32 - B);
-    const uint32_t mag = __float_as_uint(__uint_as_float(0x4B000000u | v) - 8388608.0f) >> 16;
-    return mag | (v ? sign : 0u);
-}
-
 // Four slices p of four elements as e4m3 bytes (element 0 in the lowest byte):
 // every magnitude is < 16, so the conversion is exact.
 template <int B>
@@ -194,15 +182,16 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
     return d;
 }
-// 16 bytes of slice p: 8 consecutive K values of one row, as bf16.
-template <int B>
-__device__ __forceinline__ uint4 fast_slice8(const FastElem (&x)[8], int p) {
-    uint4 v;
-    v.x = pack_bf16x2(fast_slice<B>(x[0], p), fast_slice<B>(x[1], p));
-    v.y = pack_bf16x2(fast_slice<B>(x[2], p), fast_slice<B>(x[3], p));
-    v.z = pack_bf16x2(fast_slice<B>(x[4], p), fast_slice<B>(x[5], p));
-    v.w = pack_bf16x2(fast_slice<B>(x[6], p), fast_slice<B>(x[7], p));
-    return v;
+// 16 bytes of bf16: 8 consecutive K values of one unit's slice.
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+    return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
+                      pack_bf16x2(f[6], f[7]));
+}
+__device__ __forceinline__ float sum_sq8(const float (&f)[8]) {
+    float n = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) n = fmaf(f[i], f[i], n);
+    return n;
 }
 
 __host__ __device__ inline bool split_two_windows(int b, int s) {
@@ -213,24 +202,31 @@ __host__ __device__ inline bool split_two_windows(int b, int s) {
 
 // Slices of 8 consecutive K values x of one unit (row of A or column of B) with
 // exponent E: one 16-byte piece per bf16 slice (8 bytes per e4m3 slice) at dst + p
-// slice_elems.  one_window: !split_two_windows(B, s).
-template <int B, bool F8>
+// slice_elems.  one_window: !split_two_windows(B, s).  NORM: nrm[p] += the squares of
+// slice p's values (exact: integers below 2^24).
+template <int B, bool F8, bool NORM>
 __device__ __forceinline__ void emit8(const double (&x)[8], int E, bool one_window, int s, size_t slice_elems,
-                                      uint8_t *__restrict__ dst) {
+                                      uint8_t *__restrict__ dst, float *nrm) {
     if (!F8 && one_window) {
         FastElem fe[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) fe[i] = fast_elem(x[i], E);
 #pragma unroll
         for (int p = 0; p < 64 / B; ++p)
-            if (p < s) *reinterpret_cast<uint4 *>(dst + p * slice_elems * 2) = fast_slice8<B>(fe, p);
+            if (p < s) {
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f[i] = fast_slice<B>(fe[i], p);
+                if constexpr (NORM) nrm[p] += sum_sq8(f);
+                *reinterpret_cast<uint4 *>(dst + p * slice_elems * 2) = pack8(f);
+            }
         return;
     }
     uint32_t w[8][5], sg[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) split_words(split_value(x[i], E, !one_window), w[i], sg[i]);
 #pragma unroll
-    for (int p = 0; p < 128 / B; ++p) {
+    for (int p = 0; p < (NORM ? kMaxNormSlices : 128 / B); ++p) {
         if (p < s) {
             if constexpr (F8) {
                 uint2 v;
@@ -238,13 +234,37 @@ __device__ __forceinline__ void emit8(const double (&x)[8], int E, bool one_wind
                 v.y = slices_e4m3x4<B>(w + 4, sg + 4, p);
                 *reinterpret_cast<uint2 *>(dst + p * slice_elems) = v;
             } else {
-                uint4 v;
-                v.x = slice_bits<B>(w[0], sg[0], p) | (slice_bits<B>(w[1], sg[1], p) << 16);
-                v.y = slice_bits<B>(w[2], sg[2], p) | (slice_bits<B>(w[3], sg[3], p) << 16);
-                v.z = slice_bits<B>(w[4], sg[4], p) | (slice_bits<B>(w[5], sg[5], p) << 16);
-                v.w = slice_bits<B>(w[6], sg[6], p) | (slice_bits<B>(w[7], sg[7], p) << 16);
-                *reinterpret_cast<uint4 *>(dst + p * slice_elems * 2) = v;
+                uint32_t v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float f0 = slice_float<B>(w[2 * i], sg[2 * i], p), f1 = slice_float<B>(w[2 * i + 1], sg[2 * i + 1], p);
+                    if constexpr (NORM) nrm[p] = fmaf(f1, f1, fmaf(f0, f0, nrm[p]));
+                    v[i] = pack_bf16x2(f0, f1);
+                }
+                *reinterpret_cast<uint4 *>(dst + p * slice_elems * 2) = make_uint4(v[0], v[1], v[2], v[3]);
             }
+        }
+    }
+}
+
+// The largest of the warp's chunk sums of squares per slice into the tile's maxima (bit
+// patterns of non-negative floats order like integers): tiles t0 and, for lanes whose
+// unit lies in the next tile, t0 + 1.
+__device__ __forceinline__ void norm_max(const float *nrm, int s, float *__restrict__ out, int t0, int t) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        if (!__any_sync(0xffffffffu, t == t0 + d)) continue;
+        uint32_t mine = 0;
+#pragma unroll
+        for (int p = 0; p < kMaxNormSlices; ++p)
+            if (p < s) {
+                const uint32_t v = __reduce_max_sync(0xffffffffu, t == t0 + d ? __float_as_uint(nrm[p]) : 0u);
+                if (lane == p) mine = v;
+            }
+        if (lane < s) {
+            uint32_t *at = reinterpret_cast<uint32_t *>(out) + static_cast<size_t>(t0 + d) * s + lane;
+            if (mine > __ldcg(at)) atomicMax(at, mine);
         }
     }
 }
@@ -276,60 +296,102 @@ __device__ __forceinline__ void load8(const double *__restrict__ src, int n, dou
 
 // A [M][K] row-major -> A slice blocks [mt][c][p][128 x KC].  One thread takes 8
 // consecutive K values of one row and writes one 16-byte piece per slice; a warp
-// covers 8 rows x 32 K (4 core matrices of each slice, 512 contiguous bytes).
-template <int B, bool F8 = false>
+// covers 8 rows x 32 K (4 core matrices of each slice, 512 contiguous bytes).  NORM:
+// the chunk's sums of squares are the sums over the lanes of a row (KC = 16 or 32).
+template <int B, bool F8 = false, bool NORM = false>
 __device__ __forceinline__ void split_a_body(const double *__restrict__ A, long lda, int M, int K,
                                              const int32_t *__restrict__ er, int s, int KC, int n_kc, int Mp,
-                                             uint16_t *__restrict__ tiles, int bx, int by, bool trans) {
+                                             uint16_t *__restrict__ tiles, int bx, int by, bool trans,
+                                             float *__restrict__ norm = nullptr) {
     const int r8 = threadIdx.x & 7;
     const int kgl = threadIdx.x >> 3;  // 0..31
     const int m = by * 8 + r8;
     const int k0 = (bx * 32 + kgl) * 8;
     const int Kp = n_kc * KC;
-    if (m >= Mp || k0 >= Kp) return;
-    double x[8];
-    if (!trans) {
-        load8(A + static_cast<size_t>(m) * lda + k0, m < M ? K - k0 : 0, x);
-    } else {
+    float nrm[NORM ? kMaxNormSlices : 1];
+    if constexpr (NORM) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            x[i] = (m < M && k0 + i < K) ? __ldg(A + static_cast<size_t>(k0 + i) * lda + m) : 0.0;
+        for (int p = 0; p < kMaxNormSlices; ++p) nrm[p] = 0.0f;
     }
-    emit8<B, F8>(x, m < M ? er[m] : 0, !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
-                 slice_dst<F8>(tiles, m, k0, BM, KC, n_kc, s));
+    if (m < Mp && k0 < Kp) {
+        double x[8];
+        if (!trans) {
+            load8(A + static_cast<size_t>(m) * lda + k0, m < M ? K - k0 : 0, x);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                x[i] = (m < M && k0 + i < K) ? __ldg(A + static_cast<size_t>(k0 + i) * lda + m) : 0.0;
+        }
+        emit8<B, F8, NORM>(x, m < M ? er[m] : 0, !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
+                           slice_dst<F8>(tiles, m, k0, BM, KC, n_kc, s), nrm);
+    }
+    if constexpr (NORM) {
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < kMaxNormSlices; ++p)
+            if (p < s) {
+                nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 8);
+                if (KC == 32) nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 16);
+            }
+        if (by * 8 < Mp) norm_max(nrm, s, norm, (by * 8) / BM, (by * 8) / BM);
+    }
 }
-template <int B, bool F8>
+template <int B, bool F8, bool NORM = false>
 __global__ void k_split_a(const double *__restrict__ A, long lda, int M, int K, const int32_t *__restrict__ er,
-                          int s, int KC, int n_kc, int Mp, uint16_t *__restrict__ tiles, int trans) {
-    split_a_body<B, F8>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, blockIdx.x, blockIdx.y, trans != 0);
+                          int s, int KC, int n_kc, int Mp, uint16_t *__restrict__ tiles, int trans,
+                          float *__restrict__ norm) {
+    split_a_body<B, F8, NORM>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, blockIdx.x, blockIdx.y, trans != 0, norm);
 }
 
 // B [K][N] row-major -> slice blocks of B^T [nt][c][q][BN x KC].  One thread
 // takes one column n and 8 consecutive K; a warp reads 32 consecutive columns
-// per row (coalesced) and writes four 128-byte core matrices per slice.
-template <int B, bool F8 = false>
+// per row (coalesced) and writes four 128-byte core matrices per slice.  NORM: one
+// thread takes all KC (16 or 32) values of its column's chunk, 8 at a time, so that the
+// chunk's sums of squares are its own.
+template <int B, bool F8 = false, bool NORM = false>
 __device__ __forceinline__ void split_b_body(const double *__restrict__ Bm, long ldb, int K, int N,
                                              const int32_t *__restrict__ ec, int s, int KC, int n_kc, int BN, int Np,
-                                             uint16_t *__restrict__ tiles, int bx, int by, bool trans) {
+                                             uint16_t *__restrict__ tiles, int bx, int by, bool trans,
+                                             float *__restrict__ norm = nullptr) {
     const int n = bx * 32 + (threadIdx.x & 31);
-    const int k0 = (by * 8 + (threadIdx.x >> 5)) * 8;
+    const int groups = NORM ? KC >> 3 : 1;
+    const int kw = (by * 8 + (threadIdx.x >> 5)) * 8 * groups;
     const int Kp = n_kc * KC;
-    if (n >= Np || k0 >= Kp) return;
-    double x[8];
+    if (kw >= Kp) return;  // whole warps
+    float nrm[NORM ? kMaxNormSlices : 1];
+    if constexpr (NORM) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int k = k0 + i;
-        x[i] = (n < N && k < K) ? __ldg(trans ? Bm + static_cast<size_t>(n) * ldb + k : Bm + static_cast<size_t>(k) * ldb + n)
-                                : 0.0;
+        for (int p = 0; p < kMaxNormSlices; ++p) nrm[p] = 0.0f;
     }
-    emit8<B, F8>(x, n < N ? ec[n] : 0, !split_two_windows(B, s), s, static_cast<size_t>(BN) * KC,
-                 slice_dst<F8>(tiles, n, k0, BN, KC, n_kc, s));
+    if (n < Np) {
+        const int E = n < N ? ec[n] : 0;
+#pragma unroll 1
+        for (int k0 = kw; k0 < kw + 8 * groups; k0 += 8) {
+            double x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int k = k0 + i;
+                x[i] = (n < N && k < K)
+                           ? __ldg(trans ? Bm + static_cast<size_t>(n) * ldb + k : Bm + static_cast<size_t>(k) * ldb + n)
+                           : 0.0;
+            }
+            emit8<B, F8, NORM>(x, E, !split_two_windows(B, s), s, static_cast<size_t>(BN) * KC,
+                               slice_dst<F8>(tiles, n, k0, BN, KC, n_kc, s), nrm);
+        }
+    }
+    if constexpr (NORM) {
+        __syncwarp();
+        // 32 columns from a multiple of 32 on span at most two tiles
+        const int t0 = (bx * 32) / BN;
+        norm_max(nrm, s, norm, t0, n < Np ? n / BN : -1);
+    }
 }
-template <int B, bool F8>
+template <int B, bool F8, bool NORM = false>
 __global__ void k_split_b(const double *__restrict__ Bm, long ldb, int K, int N, const int32_t *__restrict__ ec,
-                          int s, int KC, int n_kc, int BN, int Np, uint16_t *__restrict__ tiles, int trans) {
+                          int s, int KC, int n_kc, int BN, int Np, uint16_t *__restrict__ tiles, int trans,
+                          float *__restrict__ norm) {
     grid_launch_dependents();
-    split_b_body<B, F8>(Bm, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, blockIdx.x, blockIdx.y, trans != 0);
+    split_b_body<B, F8, NORM>(Bm, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, blockIdx.x, blockIdx.y, trans != 0, norm);
 }
 
 // ------------------------------------------- stages (a) and (b) in one launch
@@ -347,8 +409,9 @@ struct ExpSplitJob {
     int rows;              // units are rows of X (1) or columns (0)
     int32_t *e_out;
     uint16_t *tiles;
+    float *norm;
 };
-template <int B, bool F8>
+template <int B, bool F8, bool NORM>
 __device__ __forceinline__ void exp_split_body(const ExpSplitJob &j, int s, int KC, int n_kc, int bx) {
     const int Kp = n_kc * KC;
     const bool one = !split_two_windows(B, s);
@@ -371,11 +434,35 @@ __device__ __forceinline__ void exp_split_body(const ExpSplitJob &j, int s, int 
         __syncthreads();
         const int r8 = threadIdx.x & 7, u = bx * 8 + r8;
         const int E = sh_e[r8];
-        for (int k0 = (threadIdx.x >> 3) * 8; k0 < Kp; k0 += 256) {
-            double x[8];
-            load8(j.X + static_cast<size_t>(u) * j.ld + k0, u < j.units ? j.K - k0 : 0, x);
-            emit8<B, F8>(x, E, one, s, slice_elems, slice_dst<F8>(j.tiles, u, k0, j.TB, KC, n_kc, s));
+        float top[NORM ? kMaxNormSlices : 1];
+        if constexpr (NORM) {
+#pragma unroll
+            for (int p = 0; p < kMaxNormSlices; ++p) top[p] = 0.0f;
         }
+        for (int kb = 0; kb < Kp; kb += 256) {
+            const int k0 = kb + (threadIdx.x >> 3) * 8;
+            float nrm[NORM ? kMaxNormSlices : 1];
+            if constexpr (NORM) {
+#pragma unroll
+                for (int p = 0; p < kMaxNormSlices; ++p) nrm[p] = 0.0f;
+            }
+            if (k0 < Kp) {
+                double x[8];
+                load8(j.X + static_cast<size_t>(u) * j.ld + k0, u < j.units ? j.K - k0 : 0, x);
+                emit8<B, F8, NORM>(x, E, one, s, slice_elems, slice_dst<F8>(j.tiles, u, k0, j.TB, KC, n_kc, s), nrm);
+            }
+            if constexpr (NORM) {
+                __syncwarp();
+#pragma unroll
+                for (int p = 0; p < kMaxNormSlices; ++p)
+                    if (p < s) {
+                        nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 8);
+                        if (KC == 32) nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 16);
+                        top[p] = fmaxf(top[p], nrm[p]);
+                    }
+            }
+        }
+        if constexpr (NORM) norm_max(top, s, j.norm, bx * 8 / j.TB, bx * 8 / j.TB);
     } else {
         __shared__ int sh_c[16][17];
         const int c = threadIdx.x & 15, kl = threadIdx.x >> 4;
@@ -391,23 +478,48 @@ __device__ __forceinline__ void exp_split_body(const ExpSplitJob &j, int s, int 
 #pragma unroll
         for (int r = 0; r < 16; ++r) E = max(E, sh_c[r][c]);
         if (kl == 0 && u < j.units) j.e_out[u] = E;
-        for (int k0 = kl * 8; k0 < Kp; k0 += 128) {
-            double x[8];
+        // NORM: a warp holds 16 K values of each column at a time; a chunk of 32 is bounded
+        // by twice the largest 16
+        float top[NORM ? kMaxNormSlices : 1];
+        if constexpr (NORM) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                x[i] = (u < j.units && k0 + i < j.K) ? __ldg(j.X + static_cast<size_t>(k0 + i) * j.ld + u) : 0.0;
-            emit8<B, F8>(x, E, one, s, slice_elems, slice_dst<F8>(j.tiles, u, k0, j.TB, KC, n_kc, s));
+            for (int p = 0; p < kMaxNormSlices; ++p) top[p] = 0.0f;
         }
+        for (int kb = 0; kb < Kp; kb += 128) {
+            const int k0 = kb + kl * 8;
+            float nrm[NORM ? kMaxNormSlices : 1];
+            if constexpr (NORM) {
+#pragma unroll
+                for (int p = 0; p < kMaxNormSlices; ++p) nrm[p] = 0.0f;
+            }
+            if (k0 < Kp) {
+                double x[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    x[i] = (u < j.units && k0 + i < j.K) ? __ldg(j.X + static_cast<size_t>(k0 + i) * j.ld + u) : 0.0;
+                emit8<B, F8, NORM>(x, E, one, s, slice_elems, slice_dst<F8>(j.tiles, u, k0, j.TB, KC, n_kc, s), nrm);
+            }
+            if constexpr (NORM) {
+                __syncwarp();
+#pragma unroll
+                for (int p = 0; p < kMaxNormSlices; ++p)
+                    if (p < s) {
+                        nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 16);
+                        top[p] = fmaxf(top[p], KC == 32 ? 2.0f * nrm[p] : nrm[p]);
+                    }
+            }
+        }
+        if constexpr (NORM) norm_max(top, s, j.norm, bx * 16 / j.TB, bx * 16 / j.TB);
     }
 }
-template <int B, bool F8>
+template <int B, bool F8, bool NORM = false>
 __global__ void __launch_bounds__(256) k_exp_split(const __grid_constant__ ExpSplitJob a,
                                                    const __grid_constant__ ExpSplitJob b, int n0, int s, int KC,
                                                    int n_kc) {
     grid_launch_dependents();
     const int bid = blockIdx.x;
-    if (bid < n0) exp_split_body<B, F8>(a, s, KC, n_kc, bid);
-    else exp_split_body<B, F8>(b, s, KC, n_kc, bid - n0);
+    if (bid < n0) exp_split_body<B, F8, NORM>(a, s, KC, n_kc, bid);
+    else exp_split_body<B, F8, NORM>(b, s, KC, n_kc, bid - n0);
 }
 
 // b (1..7) as a template argument: the slice positions become constants.
@@ -778,16 +890,20 @@ __global__ void k_knob_grouped(const KnobJob *__restrict__ jobs) {
 // Grouped stage (a)/(b): block -> job by binary search over block0[], then the
 // job's per-problem kernel body with its local block coordinates.
 // One stage job on its local block index (the per-problem kernels' bodies).
-// TRANS: the kernel also serves transposed splits (the grouped kernel does not,
-// which keeps its register count down).
-template <bool TRANS>
+// TRANS: the kernel also serves transposed splits; STAGES: 1 the jobs of stage (a), 2
+// those of stage (b), 3 both (the grouped kernels take one each, without transposes,
+// which keeps their registers down and their blocks per SM up).
+template <bool TRANS, int STAGES>
 __device__ __forceinline__ void run_stage_job(const StageJob &j, int local) {
     const int bx = local % j.gx, by = local / j.gx;
     const bool tr = TRANS && j.trans != 0;
+    if (STAGES == 1 || (STAGES == 3 && j.kind != JOB_SPLIT_A && j.kind != JOB_SPLIT_B)) {
+        if (j.kind == JOB_ROWMAX) rowmax_body(j.X, j.ld, j.rows, j.cols, j.e_out, j.ss_out, bx, by);
+        else if (j.kind == JOB_COLMAX) colmax_body(j.X, j.ld, j.rows, j.cols, 64, j.e_out, j.ss_out, bx, by);
+        else stats2d_body(j.X, j.ld, j.rows, j.cols, j.e_out, j.e_out2, j.prow, j.pcol, bx, by);
+        return;
+    }
     switch (j.kind) {
-        case JOB_ROWMAX: rowmax_body(j.X, j.ld, j.rows, j.cols, j.e_out, j.ss_out, bx, by); break;
-        case JOB_COLMAX: colmax_body(j.X, j.ld, j.rows, j.cols, 64, j.e_out, j.ss_out, bx, by); break;
-        case JOB_STATS: stats2d_body(j.X, j.ld, j.rows, j.cols, j.e_out, j.e_out2, j.prow, j.pcol, bx, by); break;
         // the transpose flag as a constant at each call site: a runtime flag would
         // compile both load paths into every split (measured 20 % slower)
         case JOB_SPLIT_A: {
@@ -857,13 +973,14 @@ __device__ __forceinline__ void run_stage_job(const StageJob &j, int local) {
 // job of a work block is found by a forward scan from the previous one (work
 // blocks only increase), so no block pays a search over all jobs, and a grouped
 // call of many small problems does not launch one block per 2048 elements.
-__global__ void __launch_bounds__(kStageThreads) k_stage_jobs(const StageJob *__restrict__ jobs,
-                                                              const int *__restrict__ block0, int n_jobs) {
+template <int STAGE>
+__global__ void __launch_bounds__(kStageThreads, STAGE == 1 ? 4 : 3)
+    k_stage_jobs(const StageJob *__restrict__ jobs, const int *__restrict__ block0, int n_jobs) {
     const int total = __ldg(block0 + n_jobs);
     int j = 0;
     for (int bid = blockIdx.x; bid < total; bid += gridDim.x) {
         while (j + 1 < n_jobs && __ldg(block0 + j + 1) <= bid) ++j;
-        run_stage_job<false>(jobs[j], bid - __ldg(block0 + j));
+        run_stage_job<false, STAGE>(jobs[j], bid - __ldg(block0 + j));
         // the statistics job's shared memory is written again by the next work block
         __syncthreads();
     }
@@ -874,8 +991,8 @@ __global__ void __launch_bounds__(kStageThreads) k_stage_pair(const __grid_const
                                                               const __grid_constant__ StageJob j1, int n0) {
     grid_launch_dependents();
     const int bid = blockIdx.x;
-    if (bid < n0) run_stage_job<true>(j0, bid);
-    else run_stage_job<true>(j1, bid - n0);
+    if (bid < n0) run_stage_job<true, 3>(j0, bid);
+    else run_stage_job<true, 3>(j1, bid - n0);
 }
 
 // Pseudo-random doubles in [-1, 1) (splitmix64 of the index): inputs for the
@@ -943,9 +1060,9 @@ void launch_stage_pair(StageJob j0, StageJob j1, void *stream) {
         k_stage_pair<<<n0 + n1, kStageThreads, 0, static_cast<cudaStream_t>(stream)>>>(j0, j1, n0);
 }
 
-void launch_stage_jobs(const StageJob *jobs, const int *block0, int n_jobs, int total_blocks, void *stream) {
-    if (total_blocks <= 0) return;
-    // resident blocks of k_stage_jobs on the current device, found once per device
+template <int STAGE>
+void launch_stage_jobs_of(const StageJob *jobs, const int *block0, int n_jobs, int total_blocks, void *stream) {
+    // resident blocks of the kernel on the current device, found once per device
     static std::atomic<int> resident[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -954,15 +1071,22 @@ void launch_stage_jobs(const StageJob *jobs, const int *block0, int n_jobs, int 
     if (grid <= 0) {
         int sms = 0, per_sm = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_jobs, kStageThreads, 0) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_jobs<STAGE>, kStageThreads, 0) != cudaSuccess ||
             per_sm <= 0)
             per_sm = 2;
         cudaGetLastError();
         grid = sms * per_sm;
         if (dev >= 0 && dev < 64) resident[dev].store(grid, std::memory_order_relaxed);
     }
-    k_stage_jobs<<<std::min(grid, total_blocks), kStageThreads, 0, static_cast<cudaStream_t>(stream)>>>(jobs, block0,
-                                                                                                      n_jobs);
+    k_stage_jobs<STAGE><<<std::min(grid, total_blocks), kStageThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        jobs, block0, n_jobs);
+}
+
+void launch_stage_jobs(int stage, const StageJob *jobs, const int *block0, int n_jobs, int total_blocks,
+                       void *stream) {
+    if (total_blocks <= 0) return;
+    if (stage == 1) launch_stage_jobs_of<1>(jobs, block0, n_jobs, total_blocks, stream);
+    else launch_stage_jobs_of<2>(jobs, block0, n_jobs, total_blocks, stream);
 }
 
 void launch_knob_grouped(const KnobJob *jobs, int n, void *stream) {
@@ -991,14 +1115,16 @@ void launch_colmax(const double *B, long ldb, int K, int N, int32_t *ec, double 
 
 void launch_exp_split(const double *A, long lda, bool ta, int M, int Mp, int32_t *er, uint16_t *at, const double *B,
                       long ldb, bool tb, int N, int Np, int BN, int32_t *ec, uint16_t *bt, int K, int b, int s, int KC,
-                      int n_kc, bool f8, void *stream) {
-    const ExpSplitJob ja{A, lda, M, Mp, K, BM, ta ? 0 : 1, er, at};
-    const ExpSplitJob jb{B, ldb, N, Np, K, BN, tb ? 1 : 0, ec, bt};
+                      int n_kc, bool f8, void *stream, float *norm_a, float *norm_b) {
+    const ExpSplitJob ja{A, lda, M, Mp, K, BM, ta ? 0 : 1, er, at, norm_a};
+    const ExpSplitJob jb{B, ldb, N, Np, K, BN, tb ? 1 : 0, ec, bt, norm_b};
     const int n0 = Mp / (ja.rows ? 8 : 16), n1 = Np / (jb.rows ? 8 : 16);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define OZ_CALL_ES(BB) k_exp_split<BB, false><<<n0 + n1, 256, 0, st>>>(ja, jb, n0, s, KC, n_kc)
 #define OZ_CALL_ES8(BB) k_exp_split<BB, true><<<n0 + n1, 256, 0, st>>>(ja, jb, n0, s, KC, n_kc)
-    if (f8) {
+    if (norm_a) {
+        k_exp_split<7, false, true><<<n0 + n1, 256, 0, st>>>(ja, jb, n0, s, KC, n_kc);
+    } else if (f8) {
         OZ_SPLIT_DISPATCH_F8(b, OZ_CALL_ES8)
     } else {
         OZ_SPLIT_DISPATCH(b, OZ_CALL_ES)
@@ -1008,13 +1134,15 @@ void launch_exp_split(const double *A, long lda, bool ta, int M, int Mp, int32_t
 }
 
 void launch_split_a(const double *A, long lda, int M, int K, const int32_t *er, int b, int s, int KC, int n_kc,
-                    int Mp, uint16_t *tiles, void *stream, bool trans, bool f8) {
+                    int Mp, uint16_t *tiles, void *stream, bool trans, bool f8, float *norm) {
     const int Kp = n_kc * KC;
     dim3 grid((Kp / 8 + 31) / 32, Mp / 8);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define OZ_CALL_A(BB) k_split_a<BB, false><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0)
-#define OZ_CALL_A8(BB) k_split_a<BB, true><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0)
-    if (f8) {
+#define OZ_CALL_A(BB) k_split_a<BB, false><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0, nullptr)
+#define OZ_CALL_A8(BB) k_split_a<BB, true><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0, nullptr)
+    if (norm) {
+        k_split_a<7, false, true><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0, norm);
+    } else if (f8) {
         OZ_SPLIT_DISPATCH_F8(b, OZ_CALL_A8)
     } else {
         OZ_SPLIT_DISPATCH(b, OZ_CALL_A)
@@ -1024,15 +1152,17 @@ void launch_split_a(const double *A, long lda, int M, int K, const int32_t *er, 
 }
 
 void launch_split_b(const double *B, long ldb, int K, int N, const int32_t *ec, int b, int s, int KC, int n_kc,
-                    int BN, int Np, uint16_t *tiles, void *stream, bool trans, bool f8) {
+                    int BN, int Np, uint16_t *tiles, void *stream, bool trans, bool f8, float *norm) {
     const int Kp = n_kc * KC;
-    dim3 grid((Np + 31) / 32, (Kp / 8 + 7) / 8);
+    dim3 grid((Np + 31) / 32, norm ? (n_kc + 7) / 8 : (Kp / 8 + 7) / 8);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define OZ_CALL_B(BB) \
-    k_split_b<BB, false><<<grid, 256, 0, st>>>(B, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, trans ? 1 : 0)
+    k_split_b<BB, false><<<grid, 256, 0, st>>>(B, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, trans ? 1 : 0, nullptr)
 #define OZ_CALL_B8(BB) \
-    k_split_b<BB, true><<<grid, 256, 0, st>>>(B, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, trans ? 1 : 0)
-    if (f8) {
+    k_split_b<BB, true><<<grid, 256, 0, st>>>(B, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, trans ? 1 : 0, nullptr)
+    if (norm) {
+        k_split_b<7, false, true><<<grid, 256, 0, st>>>(B, ldb, K, N, ec, s, KC, n_kc, BN, Np, tiles, trans ? 1 : 0, norm);
+    } else if (f8) {
         OZ_SPLIT_DISPATCH_F8(b, OZ_CALL_B8)
     } else {
         OZ_SPLIT_DISPATCH(b, OZ_CALL_B)

@@ -102,3 +102,26 @@ def test_one_launch_split_matches_two(ozlib, oracle, b, s, K, ta, tb):
     assert h.sync() == 0, h.last_error()
     h.close()
     _same(dC.cpu().numpy(), oracle.dgemm(A, B, b, s, s, 0), (b, s, K, ta, tb))
+
+
+@pytest.mark.parametrize("s,J", [(8, 8), (8, 9), (8, 15), (11, 12)])
+@pytest.mark.parametrize("M,N,K", [(140, 60, 1000), (130, 100, 3001)])
+@pytest.mark.parametrize("kind", ["largest", "half", "one_row", "zero"])
+def test_drains_that_follow_the_data(ozlib, oracle, s, J, M, N, K, kind):
+    """Operands whose digits are all 2^7 - 1 and of one sign reach the fp32 bound that the
+    drain periods are made for; operands that do so in some rows or columns of a tile
+    only, or hold zeros, get longer periods elsewhere.  Bit-exact in every case, with one
+    launch and with two for the stage kernels."""
+    A, B = oracle.gen_phi((M, K), 81, 1.0), oracle.gen_phi((K, N), 82, 1.0)
+    full = np.nextafter(1.0, 0.0)  # 53 ones: every digit 127
+    if kind == "largest":
+        A[:], B[:] = full, full
+    elif kind == "half":
+        A[: M // 2], B[:, ::2] = full, -full
+    elif kind == "one_row":
+        A[129, :], B[:, 17] = full, full
+    else:
+        A[:] = 0.0
+        A[3, 5] = 1.5
+    got, cfg = _run(ozlib, A, B, s, J)
+    _same(got, oracle.dgemm(A, B, 7, s, J, 0), (cfg, kind))
