@@ -693,7 +693,7 @@ struct GroupLaunch {
 
 // The launch-level fields of a plan's GemmArgs as a fixed array (no allocation):
 // problems with equal arrays share a grouped launch.
-constexpr int kLaunchFields = 16 + kMaxAcc + 4 * kMaxGroups;
+constexpr int kLaunchFields = 18 + kMaxAcc + 4 * kMaxGroups;
 struct LaunchFields {
     long long v[kLaunchFields];
     int n = 0;
@@ -701,9 +701,9 @@ struct LaunchFields {
 };
 LaunchFields launch_fields(const GemmArgs &g, const Plan &p) {
     LaunchFields f;
-    const long long head[16] = {reinterpret_cast<long long>(p.fn), static_cast<long long>(p.smem), g.KC, g.s, g.J,
+    const long long head[18] = {reinterpret_cast<long long>(p.fn), static_cast<long long>(p.smem), g.KC, g.s, g.J,
                                 g.b, g.out_mode, g.stages, g.stage_bytes, g.a_block_bytes, g.b_block_bytes,
-                                g.tmem_cols, g.n_acc, g.n_iss, g.G, g.dbl_mask};
+                                g.tmem_cols, g.n_acc, g.n_iss, g.G, g.dbl_mask, g.parts, g.part_slices};
     for (long long x : head) f.v[f.n++] = x;
     for (int a = 0; a < kMaxAcc; ++a) f.v[f.n++] = g.acc_t0[a];
     for (int i = 0; i < g.G; ++i)

@@ -339,9 +339,18 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + static_cast<size_t>(g.stages) * g.stage_bytes);
+    // A in parts (e4m3 plans whose slices fill shared memory, GemmArgs::parts): a ring of
+    // A parts and one of two B blocks; otherwise a ring of stages that hold both
+    const int parts = F8 ? g.parts : 1;
+    const uint32_t a_stride = parts > 1 ? g.part_bytes : g.stage_bytes;
+    const uint32_t b_base = parts > 1 ? static_cast<uint32_t>(g.stages) * g.part_bytes : g.a_block_bytes;
+    const uint32_t b_stride = parts > 1 ? g.b_block_bytes : g.stage_bytes;
+    uint64_t *full = reinterpret_cast<uint64_t *>(
+        smem + (parts > 1 ? b_base + kPartStagesB * g.b_block_bytes : static_cast<uint32_t>(g.stages) * g.stage_bytes));
     uint64_t *empty = full + g.stages;
-    uint64_t *gfull = empty + g.stages;
+    uint64_t *fullb = empty + g.stages;  // parts > 1: the B ring
+    uint64_t *emptyb = fullb + kPartStagesB;
+    uint64_t *gfull = emptyb + kPartStagesB;
     uint64_t *gempty = gfull + 2 * kMaxGroups;  // [block][buffer]: index 2 * blk + buf
     uint64_t *mma_done = gempty + 2 * kMaxGroups;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
@@ -353,7 +362,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     // the drain warps' last two commands
     int2 *drain_cmd = reinterpret_cast<int2 *>((reinterpret_cast<uintptr_t>(split_flag + 1) + 7) & ~uintptr_t(7));
     // the issuers' UMMA lists, decoded: x = accumulator column | the block's other
-    // buffer's << 16, y = A offset | block << 16 | entries left in the block << 24,
+    // buffer's << 16, y = A offset | the block's first << 14 and last << 15 entries of the
+    // chunk | block << 16 | entries left in the block (and part) << 24,
     // z = B offset (descriptor units), w = instruction descriptor
     uint4 *recs = reinterpret_cast<uint4 *>((reinterpret_cast<uintptr_t>(drain_cmd + 2) + 15) & ~uintptr_t(15));
 
@@ -369,7 +379,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                                 : d0;
         const uint32_t idesc = (F8 ? idesc_e4m3_f32(BM, 16) : idesc_bf16_f32(BM, 16)) & ~(0x3Fu << 17);
         recs[i] = make_uint4(d0 | (d1 << 16),
-                             static_cast<uint32_t>(p) * ((BM * KC * 2) >> 4) | (static_cast<uint32_t>(blk) << 16) |
+                             static_cast<uint32_t>(p % g.part_slices) * ((BM * KC * 2) >> 4) |
+                                 (op_first(op) ? 0x4000u : 0u) | (op_last(op) ? 0x8000u : 0u) | (static_cast<uint32_t>(blk) << 16) |
                                  (static_cast<uint32_t>(op_left(op)) << 24),
                              static_cast<uint32_t>(lo - p) * ((BN * KC * 2) >> 4),
                              idesc | (static_cast<uint32_t>((nb * BN) >> 3) << 17));
@@ -378,6 +389,10 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         for (int i = 0; i < g.stages; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], n_iss);
+        }
+        for (int i = 0; i < kPartStagesB; ++i) {
+            mbar_init(&fullb[i], 1);
+            mbar_init(&emptyb[i], n_iss);
         }
         for (int i = 0; i < g.G; ++i) {
             for (int b = 0; b < 2; ++b) {
@@ -431,42 +446,61 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
       if (warp == 0) {
         // ------------------------------------------------------ producer
         if (lane == 0) {
-            long long issued = 0;  // stage uses by this CTA over all of its tiles
-            int st = 0;
+            // uses of the ring's entries (and of the B ring's) by this CTA over all of its tiles
+            long long issued = 0, issued_b = 0;
             bool ok = true;
-            // waits until stage st may be refilled: use r (>= 1) of a stage waits for
-            // the (r-1)-th release of that stage
-            auto acquire = [&]() -> bool {
-                const long long r = issued / g.stages;
-                const bool got = (r == 0) || mbar_wait(&empty[st], static_cast<uint32_t>((r - 1) & 1), vabort, TO);
+            // waits until the next entry of a ring may be refilled: its use r (>= 1) waits for
+            // the entry's release r - 1
+            auto acquire = [&](uint64_t *released, long long uses, int n) -> int {
+                const long long r = uses / n;
+                const int e = static_cast<int>(uses - r * n);
+                const bool got = (r == 0) || mbar_wait(&released[e], static_cast<uint32_t>((r - 1) & 1), vabort, TO);
                 if (!got && !*vabort) {
                     atomicCAS(g.err, 0, DEVERR_TIMEOUT_PRODUCER);
                     *vabort = 1;
                 }
-                return got;
+                return got ? e : -1;
             };
             for (int t = g.tile_begin + static_cast<int>(blockIdx.x); ok && t < g.total_tiles; t += gridDim.x) {
                 TileRef tr;
                 tile_ref(g, t, &tr);
-                for (int c = tr.c0; c < tr.c1; ++c) {
-                    if (*vabort || !acquire()) {
-                        ok = false;
-                        break;
+                for (int c = tr.c0; ok && c < tr.c1; ++c) {
+                    const uint8_t *a_src = tr.a_src + static_cast<size_t>(c) * g.a_block_bytes;
+                    const uint8_t *b_src = tr.b_src + static_cast<size_t>(c) * g.b_block_bytes;
+                    if (parts > 1) {
+                        const int sb = *vabort ? -1 : acquire(emptyb, issued_b, kPartStagesB);
+                        if (sb < 0) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect_tx(&fullb[sb], g.b_block_bytes);
+                        bulk_g2s(smem + b_base + static_cast<uint32_t>(sb) * b_stride, b_src, g.b_block_bytes, &fullb[sb]);
+                        ++issued_b;
                     }
-                    uint8_t *dst = smem + static_cast<size_t>(st) * g.stage_bytes;
-                    mbar_arrive_expect_tx(&full[st], g.a_block_bytes + g.b_block_bytes);
-                    bulk_g2s(dst, tr.a_src + static_cast<size_t>(c) * g.a_block_bytes, g.a_block_bytes, &full[st]);
-                    bulk_g2s(dst + g.a_block_bytes, tr.b_src + static_cast<size_t>(c) * g.b_block_bytes, g.b_block_bytes,
-                             &full[st]);
-                    ++issued;
-                    if (++st == g.stages) st = 0;
+                    uint32_t left = g.a_block_bytes;
+                    for (int i = 0; i < parts; ++i) {
+                        const int st = *vabort ? -1 : acquire(empty, issued, g.stages);
+                        if (st < 0) {
+                            ok = false;
+                            break;
+                        }
+                        uint8_t *dst = smem + static_cast<size_t>(st) * a_stride;
+                        const uint32_t bytes = parts > 1 ? min(left, g.part_bytes) : left;
+                        mbar_arrive_expect_tx(&full[st], bytes + (parts > 1 ? 0u : g.b_block_bytes));
+                        bulk_g2s(dst, a_src, bytes, &full[st]);
+                        if (parts == 1) bulk_g2s(dst + g.a_block_bytes, b_src, g.b_block_bytes, &full[st]);
+                        a_src += bytes;
+                        left -= bytes;
+                        ++issued;
+                    }
                 }
             }
             // every copy issued must land before the CTA may exit
             const int zero = 0;
-            const long long first = issued - g.stages;
-            for (long long c = (first > 0 ? first : 0); c < issued; ++c)
-                mbar_wait(&full[c % g.stages], static_cast<uint32_t>((c / g.stages) & 1), &zero, TO);
+            for (long long u = issued > g.stages ? issued - g.stages : 0; u < issued; ++u)
+                mbar_wait(&full[u % g.stages], static_cast<uint32_t>((u / g.stages) & 1), &zero, TO);
+            for (long long u = issued_b > kPartStagesB ? issued_b - kPartStagesB : 0; u < issued_b; ++u)
+                mbar_wait(&fullb[u % kPartStagesB], static_cast<uint32_t>((u / kPartStagesB) & 1), &zero, TO);
         }
       } else {
         // ---------------------------------------------------- MMA issuers
@@ -486,10 +520,12 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
             // descriptors of stage 0's A and B; the address is in the low word, and
             // adding offsets never carries out of its 14 bits
             const uint32_t a0 = smem_u32(smem);
-            const uint64_t ad0 = smem_desc(a0, 128, sbo), bd0 = smem_desc(a0 + g.a_block_bytes, 128, sbo);
+            const uint64_t ad0 = smem_desc(a0, 128, sbo), bd0 = smem_desc(a0 + b_base, 128, sbo);
             const uint32_t a_lo = static_cast<uint32_t>(ad0), b_lo = static_cast<uint32_t>(bd0);
             const uint64_t d_hi = ad0 & 0xFFFFFFFF00000000ull;
-            const int r0 = iss ? g.op_end[iss - 1] : 0, r1 = g.op_end[iss];
+            const int list0 = iss ? g.op_end[iss - 1] : 0;
+            int stb = 0;             // B ring
+            uint32_t bparity = 0;
             uint32_t ephase = 0;   // parity of the gempty waits, bit 2 blk + buf
             uint32_t pend = 0;     // drains committed and not yet waited for, bit 2 blk + buf
             uint32_t bufm = 0;     // accumulator buffer each block writes now
@@ -510,21 +546,31 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                         if (c == tr.c1 - 1) cur = (1u << g.G) - 1u;
                         else till = step = ds.next(tr.c1 - 1 - c);
                     }
+                    if (parts > 1 && !__all_sync(0xffffffffu, mbar_wait(&fullb[stb], bparity, vabort, TO))) {
+                        ok = false;
+                        break;
+                    }
+                    int r0 = list0;
+                    for (int part = 0; part < parts; ++part) {
+                    const int r1 = parts > 1 ? g.part_end[iss * kMaxParts + part] : g.op_end[iss];
                     if (!__all_sync(0xffffffffu, mbar_wait(&full[st], fparity, vabort, TO))) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t soff = (static_cast<uint32_t>(st) * g.stage_bytes) >> 4;
+                    const uint32_t soff = (static_cast<uint32_t>(st) * a_stride) >> 4;
+                    const uint32_t boff = (static_cast<uint32_t>(parts > 1 ? stb : st) * b_stride) >> 4;
                     for (int i = r0; i < r1;) {
-                        // one block: its list ends where the first entry's count says
+                        // one block (of this part): its list ends where the first entry's count says
                         uint4 rc[4];
 #pragma unroll
                         for (int x = 0; x < 4; ++x) rc[x] = recs[min(i + x, r1 - 1)];
                         const uint32_t blk = (rc[0].y >> 16) & 0xFu;
                         const int end = i + static_cast<int>(rc[0].y >> 24);
                         const uint32_t buf = (bufm >> blk) & 1u, ix = 2 * blk + buf;
-                        if ((pend >> ix) & 1u) {
+                        // with parts, the block's first and last entries of the chunk are marked
+                        const bool first = parts == 1 || (rc[0].y & 0x4000u), last = parts == 1 || (rc[0].y & 0x8000u);
+                        if (first && ((pend >> ix) & 1u)) {
                             // the buffer's previous drain must have read it out
                             if (!__all_sync(0xffffffffu, mbar_wait(&gempty[ix], (ephase >> ix) & 1u, vabort, TO))) {
                                 ok = false;
@@ -535,15 +581,15 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                             tc_fence_after();
                         }
                         // a drained block's first UMMA spans the block and overwrites it
-                        uint32_t acc0 = ((fresh & ~g.zero_mask) >> blk & 1u) ^ 1u;
+                        uint32_t acc0 = first ? ((fresh & ~g.zero_mask) >> blk & 1u) ^ 1u : 1u;
                         fresh &= ~(1u << blk);
                         while (true) {
                             if (elect_one()) {
 #pragma unroll
                                 for (int x = 0; x < 4; ++x) {
                                     const uint32_t d = tmem + (buf ? rc[x].x >> 16 : rc[x].x & 0xFFFFu);
-                                    const uint64_t ad = d_hi | (a_lo + soff + (rc[x].y & 0xFFFFu));
-                                    const uint64_t bd = d_hi | (b_lo + soff + rc[x].z);
+                                    const uint64_t ad = d_hi | (a_lo + soff + (rc[x].y & 0x3FFFu));
+                                    const uint64_t bd = d_hi | (b_lo + boff + rc[x].z);
                                     if (x == 0 || i + x < end) {
 #pragma unroll
                                         for (int kk = 0; kk < ksteps; ++kk) {
@@ -564,7 +610,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
 #pragma unroll
                             for (int x = 0; x < 4; ++x) rc[x] = recs[min(i + x, r1 - 1)];
                         }
-                        if ((cur >> blk) & 1u) {
+                        if (last && ((cur >> blk) & 1u)) {
                             if (elect_one()) umma_commit(&gfull[ix]);
                             __syncwarp();
                             pend |= 1u << ix;
@@ -578,6 +624,17 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
                     if (++st == g.stages) {
                         st = 0;
                         fparity ^= 1u;
+                    }
+                    r0 = r1;
+                    }
+                    if (!ok) break;
+                    if (parts > 1) {
+                        if (elect_one()) umma_commit(&emptyb[stb]);
+                        __syncwarp();
+                        if (++stb == kPartStagesB) {
+                            stb = 0;
+                            bparity ^= 1u;
+                        }
                     }
                 }
             }

@@ -38,15 +38,21 @@ static_assert(32 * kEpiWarps * kDrainRegs + 32 * kCtrlWarps * kCtrlRegs <= kThre
 constexpr int kMaxIssuers = 3;
 constexpr int kMaxAccWords = 5;
 constexpr int kMaxNormSlices = 16; // slices of products whose drains follow the data (Plan::norms)
+constexpr int kMaxParts = 4;       // parts of A's slices (GemmArgs::parts)
+constexpr int kPartStagesB = 2;    // B blocks in shared memory when A comes in parts
 constexpr int kMaxOps = 384;       // UMMA list of a plan (GemmArgs::ops)
 
 // One entry of a plan's UMMA list: A slice p against the B slices of bins
 // [lo, lo + nb) of block blk, i.e. q = lo - p .. lo + nb - 1 - p, all within [0, s);
-// left: entries of the block from this one on.
-OZ_HD inline uint32_t pack_op(int p, int lo, int nb, int blk, int left) {
+// left: entries of the block (and part of A) from this one on; first, last: they are the
+// block's first or last of the chunk.
+OZ_HD inline uint32_t pack_op(int p, int lo, int nb, int blk, int left, bool first, bool last) {
     return static_cast<uint32_t>(p) | static_cast<uint32_t>(lo) << 6 | static_cast<uint32_t>(nb - 1) << 11 |
-           static_cast<uint32_t>(blk) << 16 | static_cast<uint32_t>(left) << 20;
+           static_cast<uint32_t>(blk) << 16 | static_cast<uint32_t>(left) << 20 | (first ? 1u << 28 : 0u) |
+           (last ? 1u << 29 : 0u);
 }
+OZ_HD inline bool op_first(uint32_t op) { return ((op >> 28) & 1u) != 0; }
+OZ_HD inline bool op_last(uint32_t op) { return ((op >> 29) & 1u) != 0; }
 OZ_HD inline int op_p(uint32_t op) { return static_cast<int>(op & 63u); }
 OZ_HD inline int op_lo(uint32_t op) { return static_cast<int>((op >> 6) & 31u); }
 OZ_HD inline int op_nb(uint32_t op) { return static_cast<int>((op >> 11) & 31u) + 1; }
@@ -119,6 +125,14 @@ struct GemmArgs {
     // such UMMA (more bins than slices): theirs all accumulate, and the drain warps
     // store zeros over what they read.
     int op_end[kMaxIssuers];
+    // Slices that leave room for one stage (e4m3, s > 20 or so): A comes in `parts` parts
+    // of part_slices slices, part_bytes each, through a ring of `stages` parts, B through
+    // a ring of kPartStagesB blocks, so that the copies of one chunk overlap the UMMAs of
+    // another.  The lists are then ordered by part, issuer i's part j ending at
+    // part_end[i kMaxParts + j].  parts = 1: part_slices = s.
+    int parts, part_slices;
+    uint32_t part_bytes;
+    int part_end[kMaxIssuers * kMaxParts];
     uint32_t zero_mask;
     uint32_t ops[kMaxOps];
     // Double-buffered blocks (bit g of dbl_mask): a second accumulator range at

@@ -406,46 +406,66 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     // cycles per K step at s = 8, p + q <= 8, BN = 48).  Each block belongs to one of
     // the issuing warps, dealt by cost: one thread issues a UMMA about every 60-80
     // cycles at best, more with the drain warps on its scheduler.
-    {
+    // With A in parts (of sp slices) the UMMAs of each part come together.
+    auto build_lists = [&](int sp) {
         p.n_iss = hint.issuers >= 1 && hint.issuers <= kMaxIssuers ? hint.issuers : kMaxIssuers;
         p.n_iss = std::min(p.n_iss, p.G);
-        std::vector<uint32_t> ops[kMaxGroups];
+        p.part_slices = sp;
+        p.parts = (s + sp - 1) / sp;
+        std::vector<uint32_t> ops[kMaxGroups][kMaxParts];
         double cost[kMaxGroups] = {0}, load[kMaxIssuers] = {0};
         int order[kMaxGroups], owner[kMaxGroups];
         p.mma_per_kstep = 0;
+        p.zero_mask = 0;
         for (int g = 0; g < p.G; ++g) {
             const int lo = p.blk_lo[g], hi = lo + p.blk_nb[g] - 1;
             order[g] = g;
+            int first = -1;  // the first part with UMMAs of the block
             for (int pa = 0; pa < s; ++pa) {
                 const int a = std::max(lo, pa), e = std::min(hi, pa + s - 1);
                 if (a > e) continue;
-                ops[g].push_back(pack_op(pa, a, e - a + 1, g, 0));
+                ops[g][pa / sp].push_back(pack_op(pa, a, e - a + 1, g, 0, false, false));
+                if (first < 0) first = pa / sp;
                 cost[g] += std::max(0.5 * (e - a + 1) * p.BN, 32.0 + 0.25 * (e - a + 1) * p.BN);
+                ++p.mma_per_kstep;
             }
-            const auto full = std::find_if(ops[g].begin(), ops[g].end(),
-                                           [&](uint32_t op) { return op_nb(op) == p.blk_nb[g]; });
-            if (full != ops[g].end()) std::swap(*full, ops[g].front());
+            auto &f = ops[g][first];
+            const auto full =
+                std::find_if(f.begin(), f.end(), [&](uint32_t op) { return op_nb(op) == p.blk_nb[g]; });
+            if (full != f.end()) std::swap(*full, f.front());
             else p.zero_mask |= 1u << g;
-            p.mma_per_kstep += static_cast<int>(ops[g].size());
-        }
-        if (p.mma_per_kstep > kMaxOps) {
-            *err = "too many UMMAs per K step";
-            return false;
         }
         std::stable_sort(order, order + p.G, [&](int x, int y) { return cost[x] > cost[y]; });
         for (int i = 0; i < p.G; ++i) {
             owner[order[i]] = static_cast<int>(std::min_element(load, load + p.n_iss) - load);
             load[owner[order[i]]] += cost[order[i]];
         }
+        if (p.mma_per_kstep > kMaxOps) return false;
         for (int i = 0, n = 0; i < p.n_iss; ++i) {
-            for (int g = 0; g < p.G; ++g)
-                if (owner[g] == i)
-                    for (size_t k = 0; k < ops[g].size(); ++k)
-                        p.ops[n++] = pack_op(op_p(ops[g][k]), op_lo(ops[g][k]), op_nb(ops[g][k]), g,
-                                             static_cast<int>(ops[g].size() - k));
+            for (int j = 0; j < p.parts; ++j) {
+                for (int g = 0; g < p.G; ++g) {
+                    const auto &l = ops[g][j];
+                    if (owner[g] != i || l.empty()) continue;
+                    bool first = true, last = true;
+                    for (int q = 0; q < p.parts; ++q) {
+                        first = first && (q >= j || ops[g][q].empty());
+                        last = last && (q <= j || ops[g][q].empty());
+                    }
+                    for (size_t k = 0; k < l.size(); ++k)
+                        p.ops[n++] = pack_op(op_p(l[k]), op_lo(l[k]), op_nb(l[k]), g, static_cast<int>(l.size() - k),
+                                             first, last);
+                }
+                p.part_end[i * kMaxParts + j] = n;
+            }
             p.op_end[i] = n;
         }
+        return true;
+    };
+    if (!build_lists(s)) {
+        *err = "too many UMMAs per K step";
+        return false;
     }
+
     // ---- pipeline: K chunk and stage count (a chunk of 32 bf16 or 64 e4m3 K values
     // is 64 bytes per row and slice)
     const size_t eb = p.f8 ? 1 : 2;
@@ -528,6 +548,22 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     p.b_elems = static_cast<size_t>(p.tiles_n) * p.n_kc * s * p.BN * p.KC;
     p.a_bytes = p.a_elems * eb;
     p.b_bytes = p.b_elems * eb;
+    if (p.f8 && p.stages == 1) {
+        // one stage leaves the UMMAs and the copies to take turns: A in the fewest parts
+        // that leave room for a chunk's parts and one more, beside two B blocks
+        for (int np = 2; np <= kMaxParts; ++np) {
+            const int sp = (s + np - 1) / np;
+            const size_t part = static_cast<size_t>(sp) * BM * p.KC * eb;
+            const size_t room = budget - ops_bytes - kPartStagesB * static_cast<size_t>(p.b_block_bytes);
+            if ((s + sp - 1) / sp != np || room / part < static_cast<size_t>(np) + 1) continue;
+            if (!build_lists(sp)) break;
+            p.part_bytes = static_cast<uint32_t>(part);
+            p.stages = static_cast<int>(std::min<size_t>(room / part, 8));
+            p.smem = p.stages * part + kPartStagesB * static_cast<size_t>(p.b_block_bytes) + kCtrlBytes + ops_bytes;
+            *out = p;
+            return true;
+        }
+    }
     while (p.stages > 1 && p.stages * static_cast<size_t>(p.stage_bytes) + kCtrlBytes + ops_bytes > kSmemLimit) --p.stages;
     p.smem = static_cast<size_t>(p.stages) * p.stage_bytes + kCtrlBytes + ops_bytes;
     *out = p;
@@ -565,6 +601,10 @@ void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, uns
     g->dbl_mask = p.dbl_mask;
     for (int i = 0; i < p.n_iss; ++i) g->op_end[i] = p.op_end[i];
     g->zero_mask = p.zero_mask;
+    g->parts = p.parts;
+    g->part_slices = p.part_slices;
+    g->part_bytes = p.part_bytes;
+    std::memcpy(g->part_end, p.part_end, sizeof g->part_end);
     std::memcpy(g->ops, p.ops, sizeof g->ops);
 }
 

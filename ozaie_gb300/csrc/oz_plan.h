@@ -35,6 +35,8 @@ struct Plan {
     int blk_period[kMaxGroups] = {0};
     bool norms = false;  // the split takes the slices' norms, and the drains follow them (GemmArgs::na)
     int op_end[kMaxIssuers] = {0};  // the issuers' UMMA lists (GemmArgs)
+    int parts = 1, part_slices = 0, part_end[kMaxIssuers * kMaxParts] = {0};  // A in parts (GemmArgs)
+    uint32_t part_bytes = 0;
     uint32_t zero_mask = 0;
     uint32_t ops[kMaxOps] = {0};
     int n_acc = 0, acc_t0[kMaxAcc] = {0};  // drain accumulator groups (GemmArgs)

@@ -297,7 +297,9 @@ __device__ __forceinline__ void load8(const double *__restrict__ src, int n, dou
 // A [M][K] row-major -> A slice blocks [mt][c][p][128 x KC].  One thread takes 8
 // consecutive K values of one row and writes one 16-byte piece per slice; a warp
 // covers 8 rows x 32 K (4 core matrices of each slice, 512 contiguous bytes).  NORM:
-// the chunk's sums of squares are the sums over the lanes of a row (KC = 16 or 32).
+// the chunk's sums of squares are the sums over the lanes of a row (KC = 16 or 32); a
+// block takes kNormSteps times as much of K, so that it merges its maxima once.
+constexpr int kNormSteps = 4;
 template <int B, bool F8 = false, bool NORM = false>
 __device__ __forceinline__ void split_a_body(const double *__restrict__ A, long lda, int M, int K,
                                              const int32_t *__restrict__ er, int s, int KC, int n_kc, int Mp,
@@ -306,34 +308,46 @@ __device__ __forceinline__ void split_a_body(const double *__restrict__ A, long 
     const int r8 = threadIdx.x & 7;
     const int kgl = threadIdx.x >> 3;  // 0..31
     const int m = by * 8 + r8;
-    const int k0 = (bx * 32 + kgl) * 8;
     const int Kp = n_kc * KC;
-    float nrm[NORM ? kMaxNormSlices : 1];
+    float top[NORM ? kMaxNormSlices : 1];
     if constexpr (NORM) {
 #pragma unroll
-        for (int p = 0; p < kMaxNormSlices; ++p) nrm[p] = 0.0f;
+        for (int p = 0; p < kMaxNormSlices; ++p) top[p] = 0.0f;
     }
-    if (m < Mp && k0 < Kp) {
-        double x[8];
-        if (!trans) {
-            load8(A + static_cast<size_t>(m) * lda + k0, m < M ? K - k0 : 0, x);
-        } else {
+    const int E = m < M ? er[m] : 0;
+#pragma unroll 1
+    for (int it = 0; it < (NORM ? kNormSteps : 1); ++it) {
+        const int k0 = ((bx * (NORM ? kNormSteps : 1) + it) * 32 + kgl) * 8;
+        float nrm[NORM ? kMaxNormSlices : 1];
+        if constexpr (NORM) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                x[i] = (m < M && k0 + i < K) ? __ldg(A + static_cast<size_t>(k0 + i) * lda + m) : 0.0;
+            for (int p = 0; p < kMaxNormSlices; ++p) nrm[p] = 0.0f;
         }
-        emit8<B, F8, NORM>(x, m < M ? er[m] : 0, !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
-                           slice_dst<F8>(tiles, m, k0, BM, KC, n_kc, s), nrm);
+        if (m < Mp && k0 < Kp) {
+            double x[8];
+            if (!trans) {
+                load8(A + static_cast<size_t>(m) * lda + k0, m < M ? K - k0 : 0, x);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    x[i] = (m < M && k0 + i < K) ? __ldg(A + static_cast<size_t>(k0 + i) * lda + m) : 0.0;
+            }
+            emit8<B, F8, NORM>(x, E, !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
+                               slice_dst<F8>(tiles, m, k0, BM, KC, n_kc, s), nrm);
+        }
+        if constexpr (NORM) {
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < kMaxNormSlices; ++p)
+                if (p < s) {
+                    nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 8);
+                    if (KC == 32) nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 16);
+                    top[p] = fmaxf(top[p], nrm[p]);
+                }
+        }
     }
     if constexpr (NORM) {
-        __syncwarp();
-#pragma unroll
-        for (int p = 0; p < kMaxNormSlices; ++p)
-            if (p < s) {
-                nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 8);
-                if (KC == 32) nrm[p] += __shfl_xor_sync(0xffffffffu, nrm[p], 16);
-            }
-        if (by * 8 < Mp) norm_max(nrm, s, norm, (by * 8) / BM, (by * 8) / BM);
+        if (by * 8 < Mp) norm_max(top, s, norm, (by * 8) / BM, (by * 8) / BM);
     }
 }
 template <int B, bool F8, bool NORM = false>
@@ -799,15 +813,16 @@ __device__ __forceinline__ void knob_stats_body(const KnobJob &j, const int role
     __shared__ int sh_i[32];
     __shared__ double sh_d[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int ea = 0, eb = 0;
-    if (role != 1) {
-        for (int i = threadIdx.x; i < j.M; i += blockDim.x) ea = max(ea, j.er[i]);
-        ea = block_max_int(ea, sh_i);
-    }
-    if (role != 0) {
-        for (int i = threadIdx.x; i < j.N; i += blockDim.x) eb = max(eb, j.ec[i]);
-        eb = block_max_int(eb, sh_i);
-    }
+    // every block finds the largest exponents for itself: eight loads in flight per
+    // thread (one at a time this was two thirds of the kernel's 33 us at 4096^3)
+    auto largest = [&](const int32_t *e, int n) {
+        int m = 0;
+#pragma unroll 8
+        for (int i = threadIdx.x; i < n; i += blockDim.x) m = max(m, __ldg(e + i));
+        return block_max_int(m, sh_i);
+    };
+    const int ea = role != 1 ? largest(j.er, j.M) : 0;
+    const int eb = role != 0 ? largest(j.ec, j.N) : 0;
     const int n = role == 0 ? j.M : (role == 1 ? j.N : j.K);
     const int per = (n + chunks - 1) / chunks;
     const int i0 = chunk * per, i1 = min(n, i0 + per);
@@ -974,7 +989,7 @@ __device__ __forceinline__ void run_stage_job(const StageJob &j, int local) {
 // blocks only increase), so no block pays a search over all jobs, and a grouped
 // call of many small problems does not launch one block per 2048 elements.
 template <int STAGE>
-__global__ void __launch_bounds__(kStageThreads, STAGE == 1 ? 4 : 3)
+__global__ void __launch_bounds__(kStageThreads, 3)
     k_stage_jobs(const StageJob *__restrict__ jobs, const int *__restrict__ block0, int n_jobs) {
     const int total = __ldg(block0 + n_jobs);
     int j = 0;
@@ -1141,6 +1156,7 @@ void launch_split_a(const double *A, long lda, int M, int K, const int32_t *er, 
 #define OZ_CALL_A(BB) k_split_a<BB, false><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0, nullptr)
 #define OZ_CALL_A8(BB) k_split_a<BB, true><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0, nullptr)
     if (norm) {
+        grid.x = (grid.x + kNormSteps - 1) / kNormSteps;
         k_split_a<7, false, true><<<grid, 256, 0, st>>>(A, lda, M, K, er, s, KC, n_kc, Mp, tiles, trans ? 1 : 0, norm);
     } else if (f8) {
         OZ_SPLIT_DISPATCH_F8(b, OZ_CALL_A8)

@@ -125,3 +125,15 @@ def test_drains_that_follow_the_data(ozlib, oracle, s, J, M, N, K, kind):
         A[3, 5] = 1.5
     got, cfg = _run(ozlib, A, B, s, J)
     _same(got, oracle.dgemm(A, B, 7, s, J, 0), (cfg, kind))
+
+
+@pytest.mark.parametrize("b,s,J", [(3, 25, 25), (3, 27, 27), (3, 29, 29), (2, 30, 30)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (129, 17, 33), (257, 33, 700), (300, 200, 1024)])
+def test_slices_in_parts(ozlib, oracle, b, s, J, M, N, K):
+    """Narrow slices whose stage fills shared memory come in parts of A's slices: K of
+    one chunk and of many, tiles with one and with several units per SM."""
+    A = oracle.gen_phi((M, K), 83, 1.0)
+    B = oracle.gen_phi((K, N), 84, 1.0)
+    got, cfg = _run(ozlib, A, B, s, J, bits=b)
+    assert cfg["slice_format"] == 1
+    _same(got, oracle.dgemm(A, B, b, s, J, 0), cfg)
