@@ -121,18 +121,29 @@ __device__ __forceinline__ void split_words(const SplitState &st, uint32_t (&w)[
     sign = st.neg ? 0x8000u : 0u;
 }
 
-// Four slices p of four elements as e4m3 bytes (element 0 in the lowest byte):
-// every magnitude is < 16, so the conversion is exact.
+// Slice p of an element as a signed float.
 template <int B>
-__device__ __forceinline__ float slice_float(const uint32_t (&w)[5], uint32_t sign, int p) {
+__device__ __forceinline__ uint32_t slice_digit(const uint32_t (&w)[5], int p) {
     const int pos = B * p;
     const int idx = pos >> 5, off = pos & 31;
-    const uint32_t v = __funnelshift_l(w[idx + 1], w[idx], off) >> (32 - B);
-    const float f = __uint_as_float(0x4B000000u | v) - 8388608.0f;
-    return sign ? -f : f;
+    return __funnelshift_l(w[idx + 1], w[idx], off) >> (32 - B);
 }
 template <int B>
-__device__ __forceinline__ uint32_t slices_e4m3x4(const uint32_t (*w)[5], const uint32_t *sg, int p) {
+__device__ __forceinline__ float slice_float(const uint32_t (&w)[5], uint32_t sign, int p) {
+    const float f = __uint_as_float(0x4B000000u | slice_digit<B>(w, p)) - 8388608.0f;
+    return sign ? -f : f;
+}
+// Slice p of four elements as e4m3 bytes (element 0 in the lowest byte): every
+// magnitude is < 16, so the conversion is exact.  Digits of up to 3 bits select their
+// code from the eight of 0..7 by one byte permute; signs holds 0x80 in the bytes of
+// negative elements.
+template <int B>
+__device__ __forceinline__ uint32_t slices_e4m3x4(const uint32_t (*w)[5], const uint32_t *sg, uint32_t signs, int p) {
+    if constexpr (B <= 3) {
+        const uint32_t sel = slice_digit<B>(w[0], p) | slice_digit<B>(w[1], p) << 4 | slice_digit<B>(w[2], p) << 8 |
+                             slice_digit<B>(w[3], p) << 12;
+        return __byte_perm(0x44403800u, 0x4E4C4A48u, sel) | signs;  // e4m3 of 0 1 2 3, 4 5 6 7
+    }
     uint16_t lo, hi;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;"
         : "=h"(lo)
@@ -225,13 +236,16 @@ __device__ __forceinline__ void emit8(const double (&x)[8], int E, bool one_wind
     uint32_t w[8][5], sg[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) split_words(split_value(x[i], E, !one_window), w[i], sg[i]);
+    uint32_t signs[2] = {0, 0};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) signs[i >> 2] |= (sg[i] ? 0x80u : 0u) << (8 * (i & 3));
 #pragma unroll
     for (int p = 0; p < (NORM ? kMaxNormSlices : 128 / B); ++p) {
         if (p < s) {
             if constexpr (F8) {
                 uint2 v;
-                v.x = slices_e4m3x4<B>(w, sg, p);
-                v.y = slices_e4m3x4<B>(w + 4, sg + 4, p);
+                v.x = slices_e4m3x4<B>(w, sg, signs[0], p);
+                v.y = slices_e4m3x4<B>(w + 4, sg + 4, signs[1], p);
                 *reinterpret_cast<uint2 *>(dst + p * slice_elems) = v;
             } else {
                 uint32_t v[4];
