@@ -71,15 +71,16 @@ typedef struct {
     int rounding;    /* ozgb_rounding */
     int tile_n;      /* BN of the slice-pair GEMM */
     int k_chunk;     /* K elements per pipeline stage */
-    int stages;      /* pipeline stages */
-    int drain_chunks;/* K chunks accumulated in fp32 before a drain (exactness period) */
+    int stages;      /* pipeline stages (entries of the A ring when A comes in parts) */
+    int drain_chunks;/* K chunks accumulated in fp32 before a drain, for the worst case of the
+                      * digits (exactness period; larger products drain by their own digits) */
     int acc_words;   /* 32-bit words of the exact per-element accumulator */
     int pairs;       /* slice-pair products per K step */
     int blocks;      /* bin blocks (one UMMA accumulator range each) */
     int umma_per_kstep; /* UMMAs per 16-deep K step */
     int block_lo[8]; /* first bin of each block */
     int block_nb[8]; /* bins in each block */
-    int issuers;     /* warps issuing the UMMAs (1 to 3; the UMMA runs of a K step dealt round-robin) */
+    int issuers;     /* warps issuing the UMMAs (1 to 3, each those of its own bin blocks) */
     int slice_format;/* 0: bf16 slices (kind::f16); 1: e4m3 slices (kind::f8f6f4, b <= 4) */
     int dbl_blocks;  /* bit g: block g has two accumulator ranges, its UMMAs go on while one drains */
 } ozgb_config;
@@ -211,7 +212,8 @@ ozgb_status ozgb_set_grouped_launch(ozgb_handle h, int mode);
 ozgb_status ozgb_set_timeout_ms(ozgb_handle h, double ms); /* device-side wait limit, default 2000 */
 ozgb_status ozgb_get_config(ozgb_handle h, ozgb_config *out);
 /* Per-stage device times of the last call (ms): [0] exponents, [1] split,
- * [2] slice-pair GEMM + accumulation, [3] total.  Needs ozgb_set_profiling(h, 1). */
+ * [2] slice-pair GEMM + accumulation, [3] total.  Needs ozgb_set_profiling(h, 1).
+ * Small products take exponents and split in one launch, counted under [1]. */
 ozgb_status ozgb_set_profiling(ozgb_handle h, int enable);
 ozgb_status ozgb_stage_times(ozgb_handle h, float *ms, int n);
 /* Number of kernels this handle has launched so far (all entry points).  No

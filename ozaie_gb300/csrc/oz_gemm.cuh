@@ -29,7 +29,8 @@
 //   * Each block belongs to one issuing warp, so its UMMAs run in order and the
 //     first one after a drain overwrites the accumulator.  Issuers do not wait for
 //     one another beyond the stage ring.
-//   * Each block is a drain group with its own period (its tightest bin).  A block
+//   * Each block is a drain group with its own period: its tightest bin's, or longer
+//     where the norms of the tile's slices allow it (DrainSchedule).  A block
 //     whose accumulator is being read out holds up its own issuer only; a
 //     double-buffered block switches ranges at each drain instead.
 //   * Drain (warps 4..19): TMEM -> registers, fp32 -> int32 (exact), then one
@@ -46,9 +47,11 @@
 //   * Every mbarrier wait is bounded (globaltimer); on expiry the kernel records
 //     an error code, waits for its own copies and MMAs, frees TMEM and returns.
 //
-// At 4096^3 (s = 8, p + q <= 8, 2752 tiles of 128 x 48) the launch takes 3.7 ms:
-// 1600 cycles per K step of a tile, of which the UMMAs need 1104.  Without drains it
-// takes 1280; the rest is the issuers and drain warps sharing the schedulers.
+// At 4096^3 (s = 8, p + q <= 8, 2752 tiles of 128 x 48) the launch takes 3.29 ms (1790
+// TFLOP/s of slice-pair products): 1430 cycles per K step of a tile, of which the UMMAs
+// need 1104.  Without drains it takes 1280; the rest is the issuers and drain warps sharing
+// the schedulers.  (1769 cycles before: UMMAs over whole blocks, 1224 cycles a K step with
+// their zero slices, and drains by the worst case.)
 #pragma once
 #include <cuda_runtime.h>
 

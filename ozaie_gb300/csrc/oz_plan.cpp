@@ -258,16 +258,15 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     p.n_acc = n_acc;
     for (int a = 0; a < kMaxAcc; ++a) p.acc_t0[a] = acc_t0[a];
 
-    // ---- bin blocks: contiguous bin ranges of at most 256 columns; every UMMA of a
-    // block spans the whole block (zero B slices pad the out-of-range q).  Cost of
-    // a partition per 16-deep K step of a tile, in SM cycles, fitted to GB300
-    // measurements of the kernel (three issuing warps, tests/perf/umma_cost.cu for
-    // the UMMA itself): each UMMA N / 2 + 20 (the tensor pipe takes half a cycle per
-    // column; the A tile is re-read from shared memory for every UMMA), each block
-    // 200 (per-block issue work), and for each block the part of its drain (500 +
-    // 800 per 48 columns: the F2I conversions run at 16 per cycle per SM) that two
-    // K steps of the other blocks' UMMAs do not cover, once per drain period.  The
-    // search enumerates the compositions of the bins into G <= 8 blocks whose sizes
+    // ---- bin blocks: contiguous bin ranges of at most 256 columns, the drain groups.
+    // Cost of a partition per 16-deep K step of a tile, in SM cycles: each UMMA N / 2 + 20
+    // with N the block's full width, each block 200, and for each block the part of its
+    // drain (500 + 800 per 48 columns) that two K steps of the other blocks' UMMAs do not
+    // cover, once per drain period.  The model was fitted to an earlier kernel, whose UMMAs
+    // spanned whole blocks, and stays as it is: choose_schedule ranks the slice schedules by
+    // it, so it decides which bits the knob returns.  Its partitions are still within 2 % of
+    // the best measured (4096^3, s = 8, p + q <= 8: {3,3,3} 3.29 ms, {4,3,2} and {4,5} 3.35).
+    // The search enumerates the compositions of the bins into G <= 8 blocks whose sizes
     // stay within one of the even split, for every G.
     const int max_groups = kMaxGroups;
     const int maxb = 256 / p.BN;

@@ -137,3 +137,42 @@ def test_slices_in_parts(ozlib, oracle, b, s, J, M, N, K):
     got, cfg = _run(ozlib, A, B, s, J, bits=b)
     assert cfg["slice_format"] == 1
     _same(got, oracle.dgemm(A, B, b, s, J, 0), cfg)
+
+
+@pytest.mark.parametrize("M,N,K,mode", [(96, 80, 200, 1), (256, 256, 2048, 1), (2304, 2000, 600, 0)])
+def test_captured_call_replays(ozlib, M, N, K, mode):
+    """A warmed-up call captured in a CUDA graph (one stage launch and two, with and
+    without norms, the GEMM as a programmatic dependent) replays on new operands."""
+    import torch
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(5)
+    dA = torch.randn((M, K), dtype=torch.float64, device=dev, generator=gen)
+    dB = torch.randn((K, N), dtype=torch.float64, device=dev, generator=gen)
+    dC = torch.zeros((M, N), dtype=torch.float64, device=dev)
+    h = ozlib.Handle()
+    assert h.setup(M, N, K, mode) == 0, h.last_error()
+
+    def call():
+        rc = h.dgemm_device(M, N, K, dA.data_ptr(), K, dB.data_ptr(), N, dC.data_ptr(), N,
+                            torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, h.last_error()
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        call()
+    for seed in (6, 7):
+        gen.manual_seed(seed)
+        dA.normal_(generator=gen)
+        dB.normal_(generator=gen)
+        dC.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        got = dC.clone()
+        call()
+        assert h.sync() == 0, h.last_error()
+        assert torch.equal(got, dC)
+    h.close()
