@@ -409,6 +409,11 @@ struct HostOut {
     bool copied;  // set when the split path has enqueued every copy of C
 };
 
+// Bytes of the slices' norms (Plan::norms): s floats per tile of A, then of B.
+size_t norm_bytes(const Plan &p) {
+    return sizeof(float) * p.cfg.s * (static_cast<size_t>(p.tiles_m) + p.tiles_n);
+}
+
 // Stages (b) and (c)+(d) for one problem whose exponents are in h->er / h->ec, or with
 // exponents = true stage (a) too.
 ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, int out_mode, int32_t *raw,
@@ -422,7 +427,7 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
     const double elems = static_cast<double>(p.Mp + p.Np) * p.n_kc * p.KC;
     float *na = nullptr, *nb = nullptr;
     if (p.norms) {
-        const size_t bytes = sizeof(float) * p.cfg.s * (static_cast<size_t>(p.tiles_m) + p.tiles_n);
+        const size_t bytes = norm_bytes(p);
         if (!h->norm.ensure(bytes)) return fail(h, OZGB_ERR_ALLOC, "slice norms");
         cudaMemsetAsync(h->norm.p, 0, bytes, st);
         na = static_cast<float *>(h->norm.p);
@@ -1168,7 +1173,8 @@ ozgb_status ozgb_setup(ozgb_handle h, int M, int N, int K, int mode) {
     if (!make_plan(M, N, K, cfg, &p, &why)) return fail(h, OZGB_ERR_UNSUPPORTED, why);
     const size_t nA = static_cast<size_t>(M) * K, nB = static_cast<size_t>(K) * N, nC = static_cast<size_t>(M) * N;
     if (!h->a.ensure(nA * 8) || !h->b.ensure(nB * 8) || !h->c.ensure(nC * 8) || !h->at.ensure(p.a_bytes) ||
-        !h->bt.ensure(p.b_bytes) || !h->er.ensure(4 * M) || !h->ec.ensure(4 * N))
+        !h->bt.ensure(p.b_bytes) || !h->er.ensure(4 * M) || !h->ec.ensure(4 * N) ||
+        (p.norms && !h->norm.ensure(norm_bytes(p))))
         return fail(h, OZGB_ERR_ALLOC, "device buffers for the setup shape");
     h->M = M;
     h->N = N;
