@@ -266,6 +266,9 @@ void ozgb_tuning_clear(void);
 /* Host-only planning query (no device needed): the kernel configuration the
  * library would use for an M x N x K product with `bits`, `slices`, `bins`. */
 int ozgb_plan_query(int M, int N, int K, int bits, int slices, int bins, ozgb_config *out);
+/* Host-only planning query: 1 if a single such product drains by its own digits (its
+ * split also takes the slices' norms), 0 if by the worst case, -1 if it has no plan. */
+int ozgb_plan_data_drains(int M, int N, int K, int bits, int slices, int bins);
 /* Host-only precision knob (no device needed): the smallest slice count in
  * [2, 16] whose a-priori normwise error estimate is <= bound (16 if none), from
  * the stage-(a) statistics: row max exponent fields er and row sums of squares

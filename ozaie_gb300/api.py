@@ -281,6 +281,12 @@ def plan_query(M, N, K, bits, slices, bins):
     return None if rc else c.as_dict()
 
 
+def plan_data_drains(M, N, K, bits, slices, bins):
+    """Whether a single such product drains by its own digits (None: it has no plan)."""
+    rc = load().ozgb_plan_data_drains(M, N, K, bits, slices, bins)
+    return None if rc < 0 else bool(rc)
+
+
 def choose_slices(er, ssr, ec, ssc, K, bits, bound, sa_k=None, sb_k=None, criterion=0, tail=1e-4):
     """Host-only precision knob: (slice count, a-priori error estimate) for a
     requested bound, from the stage-(a) statistics.  sa_k / sb_k are the sums of

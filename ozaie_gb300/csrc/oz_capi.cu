@@ -1762,6 +1762,16 @@ int ozgb_plan_query(int M, int N, int K, int bits, int slices, int bins, ozgb_co
     return OZGB_OK;
 }
 
+int ozgb_plan_data_drains(int M, int N, int K, int bits, int slices, int bins) {
+    OzConfig c;
+    c.b = bits;
+    c.s = slices;
+    c.J = bins;
+    std::string why;
+    const PlanRef p = find_plan(M, N, K, c, &why);
+    return p ? (p->norms ? 1 : 0) : -1;
+}
+
 int ozgb_choose_slices(const int32_t *er, const double *ssr, int M, const int32_t *ec, const double *ssc, int N,
                        const double *sa_k, const double *sb_k, int K, int bits, double bound, double *estimate) {
     return ozgb_choose_slices_ex(er, ssr, M, ec, ssc, N, sa_k, sb_k, K, bits, bound, OZGB_CRIT_NORMWISE, 1e-4,

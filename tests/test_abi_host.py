@@ -392,3 +392,15 @@ def test_slice_schedule_prefers_fewer_umma(ozlib):
     a = ozlib.plan_query(4096, 4096, 4096, 7, s, J)
     b = ozlib.plan_query(4096, 4096, 4096, 7, st, Jt)
     assert a["umma_per_kstep"] / a["tile_n"] < b["umma_per_kstep"] / b["tile_n"]
+
+
+def test_data_drains_rule(ozlib):
+    """More than 304 tiles, more than two worst-case periods of K, 7-bit slices: one off
+    each side of the rule."""
+    c = ozlib.plan_query(4096, 4096, 4096, 7, 8, 8)
+    k = 2 * c["drain_chunks"] * c["k_chunk"]
+    assert ozlib.plan_data_drains(128, 305 * c["tile_n"], k + 1, 7, 8, 8) is True
+    assert ozlib.plan_data_drains(128, 305 * c["tile_n"], k, 7, 8, 8) is False
+    assert ozlib.plan_data_drains(128, 304 * c["tile_n"], k + 1, 7, 8, 8) is False
+    assert ozlib.plan_data_drains(4096, 4096, 4096, 6, 9, 9) is False
+    assert ozlib.plan_data_drains(0, 1, 1, 7, 8, 8) is None
