@@ -413,6 +413,18 @@ struct HostOut {
 size_t norm_bytes(const Plan &p) {
     return sizeof(float) * p.cfg.s * (static_cast<size_t>(p.tiles_m) + p.tiles_n);
 }
+// The handle's norm buffer for a plan that takes them, zeroed on the stream; both null
+// for a plan that does not.
+ozgb_status zeroed_norms(ozgb_handle h, const Plan &p, cudaStream_t st, float **na, float **nb) {
+    *na = *nb = nullptr;
+    if (!p.norms) return OZGB_OK;
+    const size_t bytes = norm_bytes(p);
+    if (!h->norm.ensure(bytes)) return fail(h, OZGB_ERR_ALLOC, "slice norms");
+    cudaMemsetAsync(h->norm.p, 0, bytes, st);
+    *na = static_cast<float *>(h->norm.p);
+    *nb = *na + static_cast<size_t>(p.cfg.s) * p.tiles_m;
+    return OZGB_OK;
+}
 
 // Stages (b) and (c)+(d) for one problem whose exponents are in h->er / h->ec, or with
 // exponents = true stage (a) too.
@@ -421,18 +433,13 @@ ozgb_status enqueue_split_gemm(ozgb_handle h, const Operands &o, const Plan &p, 
     if (!h->at.ensure(p.a_bytes) || !h->bt.ensure(p.b_bytes))
         return fail(h, OZGB_ERR_ALLOC, "slice buffers");
     uint16_t *at = static_cast<uint16_t *>(h->at.p), *bt = static_cast<uint16_t *>(h->bt.p);
+    float *na, *nb;
+    if (const ozgb_status rc = zeroed_norms(h, p, st, &na, &nb)) return rc;
     // small operands: both splits in one launch (one launch gap less); large ones
     // run the separate kernels, whose lighter register and shared-memory use
-    // measured faster (4096^3: 0.270 against 0.291 ms)
+    // measured faster (4096^3: 0.270 against 0.291 ms), and so do those with norms,
+    // which only the separate kernels and the one-launch form take
     const double elems = static_cast<double>(p.Mp + p.Np) * p.n_kc * p.KC;
-    float *na = nullptr, *nb = nullptr;
-    if (p.norms) {
-        const size_t bytes = norm_bytes(p);
-        if (!h->norm.ensure(bytes)) return fail(h, OZGB_ERR_ALLOC, "slice norms");
-        cudaMemsetAsync(h->norm.p, 0, bytes, st);
-        na = static_cast<float *>(h->norm.p);
-        nb = na + static_cast<size_t>(p.cfg.s) * p.tiles_m;
-    }
     if (exponents) {
         launch_exp_split(o.A, o.lda, o.ta, o.M, p.Mp, static_cast<int32_t *>(h->er.p), at, o.B, o.ldb, o.tb, o.N, p.Np,
                          p.BN, static_cast<int32_t *>(h->ec.p), bt, o.K, p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.f8, st, na,
@@ -1594,10 +1601,13 @@ ozgb_status ozgb_autotune(ozgb_handle h, int M, int N, int K, int bits, int slic
         if (!make_plan(M, N, K, cfg, &p, &why, 0, 1 << 30, &cands[i])) continue;
         if (!h->at.ensure(p.a_bytes) || !h->bt.ensure(p.b_bytes)) continue;
         uint16_t *at = static_cast<uint16_t *>(h->at.p), *bt = static_cast<uint16_t *>(h->bt.p);
+        // with norms where a call would take them: the drains decide between candidates
+        float *na, *nb;
+        if (zeroed_norms(h, p, st, &na, &nb)) continue;
         launch_split_a(dA, K, M, K, static_cast<int32_t *>(h->er.p), p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.Mp, at, st,
-                       false, p.f8);
+                       false, p.f8, na);
         launch_split_b(dB, N, K, N, static_cast<int32_t *>(h->ec.p), p.cfg.b, p.cfg.s, p.KC, p.n_kc, p.BN, p.Np, bt, st,
-                       false, p.f8);
+                       false, p.f8, nb);
         GemmArgs g;
         gemm_args_from_plan(&g, p, OUT_RN, static_cast<int *>(h->err.p), h->timeout_ns);
         g.a_tiles = at;
@@ -1612,6 +1622,8 @@ ozgb_status ozgb_autotune(ozgb_handle h, int M, int N, int K, int bits, int slic
         g.tiles_m = p.tiles_m;
         g.tiles_n = p.tiles_n;
         g.total_tiles = p.tiles_m * p.tiles_n;
+        g.na = na;
+        g.nb = nb;
         p.fn(g, g.total_tiles, p.smem, st);  // warm-up
         float t[3];
         for (float &ti : t) {

@@ -1,6 +1,6 @@
 """Products whose drains follow the data (the split takes the slices' norms), held bit
-for bit to the oracle on operands that reach the fp32 bound, and their buffers.  They
-have more than 304 tiles (smaller products, test_gpu_gemm_edges.py's among them, drain by
+for bit to the oracle on operands that reach the fp32 bound; their buffers, and what the
+autotuner times of them.  They have more than 304 tiles (smaller products, test_gpu_gemm_edges.py's among them, drain by
 the worst case): the shapes here have them in one direction, or in both.
 """
 import numpy as np
@@ -113,6 +113,47 @@ def test_first_call_after_setup_can_be_captured(ozlib):
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
         call(h)
+    dC.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(dC, ref)
+    h.close()
+
+
+def test_autotune_times_the_drains_that_calls_run(ozlib):
+    """The autotuner takes the norms where a call of its plan does, so that the handle holds
+    every buffer of such a call afterwards: it can be captured, with nothing allocated."""
+    import torch
+
+    from ozaie_gb300 import api
+    dev = torch.device("cuda", 0)
+    M, N, K = 2304, 2000, 2048
+    assert ozlib.plan_data_drains(M, N, K, 7, 8, 8)
+    gen = torch.Generator(device=dev).manual_seed(10)
+    dA = torch.randn((M, K), dtype=torch.float64, device=dev, generator=gen)
+    dB = torch.randn((K, N), dtype=torch.float64, device=dev, generator=gen)
+    dC = torch.zeros((M, N), dtype=torch.float64, device=dev)
+
+    def call(h):
+        rc = h.dgemm_device(M, N, K, dA.data_ptr(), K, dB.data_ptr(), N, dC.data_ptr(), N,
+                            torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, h.last_error()
+
+    h = ozlib.Handle()  # loads the kernels
+    call(h)
+    assert h.sync() == 0, h.last_error()
+    h.close()
+    ref = dC.clone()
+    api.tuning_clear()
+    h = ozlib.Handle()
+    try:
+        h.autotune(M, N, K, 7, 8, 8, max_candidates=1)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+            call(h)
+    finally:
+        api.tuning_clear()
     dC.fill_(float("nan"))
     graph.replay()
     torch.cuda.synchronize()
