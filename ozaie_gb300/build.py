@@ -6,6 +6,7 @@ ozaie_gb300/liboz_gb300.so.  No CMake, no Triton, no torch extension machinery.
 """
 import concurrent.futures as cf
 import os
+import re
 import subprocess
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -27,7 +28,7 @@ SOURCES = [
 ]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++20", "-Xcompiler", "-fPIC", "-I", INCLUDE] + ARCH
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++20", "-Xcompiler", "-fPIC", "-Xptxas", "-v", "-I", INCLUDE] + ARCH
 
 
 def nvcc():
@@ -55,7 +56,20 @@ def _compile(src):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("nvcc failed for %s:\n%s\n%s" % (src, " ".join(cmd), r.stderr))
+    with open(os.path.splitext(obj)[0] + ".ptxas", "w") as f:  # registers, spills and shared memory of each kernel
+        f.write(r.stderr)
     return obj
+
+
+def kernel_registers(src):
+    """{mangled kernel name: registers per thread} of a translation unit, from the
+    compiler's report of the last build ({} when there is none)."""
+    path = os.path.join(BUILD, os.path.splitext(src)[0] + ".ptxas")
+    if not os.path.exists(path):
+        return {}
+    with open(path) as f:
+        text = f.read()
+    return {m[1]: int(m[2]) for m in re.finditer(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", text, re.S)}
 
 
 def build(force=False, verbose=False):

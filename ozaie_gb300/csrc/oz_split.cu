@@ -540,8 +540,12 @@ __device__ __forceinline__ void exp_split_body(const ExpSplitJob &j, int s, int 
         if constexpr (NORM) norm_max(top, s, j.norm, bx * 16 / j.TB, bx * 16 / j.TB);
     }
 }
+// NORM: two blocks per SM (128 registers, 40 bytes spilled; 146 without the bound, whose
+// one block per SM left the pass short of loads in flight: us a call, s = 8, 24000 x 64 x
+// 1500 with p + q <= 8 557 -> 435, 128 x 24000 x 400 with B transposed 264 -> 202, 2304 x
+// 2000 x 2000 516 -> 504).
 template <int B, bool F8, bool NORM = false>
-__global__ void __launch_bounds__(256) k_exp_split(const __grid_constant__ ExpSplitJob a,
+__global__ void __launch_bounds__(256, NORM ? 2 : 0) k_exp_split(const __grid_constant__ ExpSplitJob a,
                                                    const __grid_constant__ ExpSplitJob b, int n0, int s, int KC,
                                                    int n_kc) {
     grid_launch_dependents();
