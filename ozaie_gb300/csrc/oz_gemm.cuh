@@ -294,8 +294,8 @@ struct DrainSchedule {
         if (lane < g.G) period = g.blk_period[lane];
         if (tr.na) {
             // rounded up throughout; a bound of 0 (no such digits) leaves the period long
-            const float a = lane < g.s ? __fsqrt_ru(tr.na[lane]) : 0.0f;
-            const float b = lane < g.s ? __fsqrt_ru(tr.nb[lane]) : 0.0f;
+            const float a = lane < g.s ? __fsqrt_ru(ld_after_wait(tr.na + lane)) : 0.0f;
+            const float b = lane < g.s ? __fsqrt_ru(ld_after_wait(tr.nb + lane)) : 0.0f;
             float bound = 0.0f;  // of bin `lane`, per chunk
             for (int p = 0; p < g.s; ++p) {
                 const float ap = __shfl_sync(0xffffffffu, a, p);
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
 
     // everything above overlaps the end of the kernel before this one in the stream.  That
     // kernel writes the exponents, the norms and the slices: they are read below this line
-    // only, by plain loads, which the wait orders (a non-coherent load asks for data that
+    // only, by coherent loads, which the wait orders (a non-coherent load asks for data that
     // nothing writes while the kernel runs, and the wait need not order it)
     grid_wait_predecessor();
     if (threadIdx.x == 0 && *reinterpret_cast<volatile int *>(g.err) != 0) *vabort = 1;
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
             const int row = tr.mt * BM + 32 * qd + lane;
             const bool row_ok = row < tr.M;
             const int col0 = tr.nt * BN + part * COLS;
-            const int er = row_ok ? tr.er[row] : 0;
+            const int er = row_ok ? ld_after_wait(tr.er + row) : 0;
             const int e_base = er - 2044 - g.b * (g.J + 1);
             double *crow = tr.c + static_cast<size_t>(row) * tr.ldc;
             const bool plain = g.alpha == 1.0 && g.beta == 0.0;
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
 #pragma unroll
             for (int x = 0; x < kMaxAcc; ++x) B[x] = g.b * g.acc_t0[x];
             // the next pair's scale exponents are loaded a step ahead
-            auto col_exp = [&](int col) { return col < tr.N ? tr.ec[col] : 0; };
+            auto col_exp = [&](int col) { return col < tr.N ? ld_after_wait(tr.ec + col) : 0; };
             int e_next[2] = {col_exp(col0), col_exp(col0 + 1)};
 #pragma unroll 1
             for (int i = 0; i < COLS; i += 2) {
