@@ -32,6 +32,7 @@ __device__ __forceinline__ void rowmax_body(const double *__restrict__ A, long l
     const double *row = A + static_cast<size_t>(warp) * lda;
     int e = 0;
     double s2 = 0.0;
+#pragma unroll 8  // loads in flight: the loop is their latency
     for (int k = lane; k < K; k += 32) {
         const double x = __ldg(row + k);
         e = max(e, exp_field(x));
@@ -62,6 +63,7 @@ __device__ __forceinline__ void colmax_body(const double *__restrict__ B, long l
     const int k1 = min(K, k0 + rows_per_slab);
     int e = 0;
     double s2 = 0.0;
+#pragma unroll 8
     for (int k = k0; k < k1; ++k) {
         const double x = __ldg(B + static_cast<size_t>(k) * ldb + n);
         e = max(e, exp_field(x));
@@ -313,8 +315,9 @@ __device__ __forceinline__ void load8(const double *__restrict__ src, int n, dou
 // covers 8 rows x 32 K (4 core matrices of each slice, 512 contiguous bytes).  NORM:
 // the chunk's sums of squares are the sums over the lanes of a row (KC = 16 or 32); a
 // block takes kNormSteps times as much of K, so that it merges its maxima once.
+// WIN: windows of the split (split_two_windows), 0 for one or two by (B, s) at run time.
 constexpr int kNormSteps = 4;
-template <int B, bool F8 = false, bool NORM = false>
+template <int B, bool F8 = false, bool NORM = false, int WIN = 0>
 __device__ __forceinline__ void split_a_body(const double *__restrict__ A, long lda, int M, int K,
                                              const int32_t *__restrict__ er, int s, int KC, int n_kc, int Mp,
                                              uint16_t *__restrict__ tiles, int bx, int by, bool trans,
@@ -346,7 +349,7 @@ __device__ __forceinline__ void split_a_body(const double *__restrict__ A, long 
                 for (int i = 0; i < 8; ++i)
                     x[i] = (m < M && k0 + i < K) ? __ldg(A + static_cast<size_t>(k0 + i) * lda + m) : 0.0;
             }
-            emit8<B, F8, NORM>(x, E, !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
+            emit8<B, F8, NORM>(x, E, WIN ? WIN == 1 : !split_two_windows(B, s), s, static_cast<size_t>(BM) * KC,
                                slice_dst<F8>(tiles, m, k0, BM, KC, n_kc, s), nrm);
         }
         if constexpr (NORM) {
@@ -376,7 +379,7 @@ __global__ void k_split_a(const double *__restrict__ A, long lda, int M, int K, 
 // per row (coalesced) and writes four 128-byte core matrices per slice.  NORM: one
 // thread takes all KC (16 or 32) values of its column's chunk, 8 at a time, so that the
 // chunk's sums of squares are its own.
-template <int B, bool F8 = false, bool NORM = false>
+template <int B, bool F8 = false, bool NORM = false, int WIN = 0>
 __device__ __forceinline__ void split_b_body(const double *__restrict__ Bm, long ldb, int K, int N,
                                              const int32_t *__restrict__ ec, int s, int KC, int n_kc, int BN, int Np,
                                              uint16_t *__restrict__ tiles, int bx, int by, bool trans,
@@ -403,7 +406,7 @@ __device__ __forceinline__ void split_b_body(const double *__restrict__ Bm, long
                            ? __ldg(trans ? Bm + static_cast<size_t>(n) * ldb + k : Bm + static_cast<size_t>(k) * ldb + n)
                            : 0.0;
             }
-            emit8<B, F8, NORM>(x, E, !split_two_windows(B, s), s, static_cast<size_t>(BN) * KC,
+            emit8<B, F8, NORM>(x, E, WIN ? WIN == 1 : !split_two_windows(B, s), s, static_cast<size_t>(BN) * KC,
                                slice_dst<F8>(tiles, n, k0, BN, KC, n_kc, s), nrm);
         }
     }
@@ -919,17 +922,15 @@ __global__ void k_knob_grouped(const KnobJob *__restrict__ jobs) {
     knob_stats_body(j, blockIdx.x % 3, 0, 1);
 }
 
-// Grouped stage (a)/(b): block -> job by binary search over block0[], then the
-// job's per-problem kernel body with its local block coordinates.
 // One stage job on its local block index (the per-problem kernels' bodies).
-// TRANS: the kernel also serves transposed splits; STAGES: 1 the jobs of stage (a), 2
-// those of stage (b), 3 both (the grouped kernels take one each, without transposes,
-// which keeps their registers down and their blocks per SM up).
-template <bool TRANS, int STAGES>
+// TRANS: the kernel also serves transposed splits; STAGE: 1 the jobs of stage (a), 2
+// those of stage (b); WIN: 1 splits of one window (bf16), 2 the others, 0 all of them.  (A
+// kernel of fewer bodies keeps its registers down and its blocks per SM up.)
+template <bool TRANS, int STAGE, int WIN = 0>
 __device__ __forceinline__ void run_stage_job(const StageJob &j, int local) {
     const int bx = local % j.gx, by = local / j.gx;
     const bool tr = TRANS && j.trans != 0;
-    if (STAGES == 1 || (STAGES == 3 && j.kind != JOB_SPLIT_A && j.kind != JOB_SPLIT_B)) {
+    if constexpr (STAGE == 1) {
         if (j.kind == JOB_ROWMAX) rowmax_body(j.X, j.ld, j.rows, j.cols, j.e_out, j.ss_out, bx, by);
         else if (j.kind == JOB_COLMAX) colmax_body(j.X, j.ld, j.rows, j.cols, 64, j.e_out, j.ss_out, bx, by);
         else stats2d_body(j.X, j.ld, j.rows, j.cols, j.e_out, j.e_out2, j.prow, j.pcol, bx, by);
@@ -940,14 +941,14 @@ __device__ __forceinline__ void run_stage_job(const StageJob &j, int local) {
         // compile both load paths into every split (measured 20 % slower)
         case JOB_SPLIT_A: {
 #define OZ_JOB_A(BB, T) \
-    split_a_body<BB>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.padded, j.tiles, bx, by, T)
+    split_a_body<BB, false, false, WIN>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.padded, j.tiles, bx, by, T)
 #define OZ_JOB_A8(BB, T) \
-    split_a_body<BB, true>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.padded, j.tiles, bx, by, T)
+    split_a_body<BB, true, false, WIN>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.padded, j.tiles, bx, by, T)
 #define OZ_JOB_AN(BB) OZ_JOB_A(BB, false)
 #define OZ_JOB_AT(BB) OZ_JOB_A(BB, true)
 #define OZ_JOB_A8N(BB) OZ_JOB_A8(BB, false)
 #define OZ_JOB_A8T(BB) OZ_JOB_A8(BB, true)
-            if (j.f8) {
+            if (WIN != 1 && j.f8) {
                 if (tr) {
                     OZ_SPLIT_DISPATCH_F8(j.b, OZ_JOB_A8T)
                 } else {
@@ -970,14 +971,14 @@ __device__ __forceinline__ void run_stage_job(const StageJob &j, int local) {
         }
         default: {
 #define OZ_JOB_B(BB, T) \
-    split_b_body<BB>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.BN, j.padded, j.tiles, bx, by, T)
+    split_b_body<BB, false, false, WIN>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.BN, j.padded, j.tiles, bx, by, T)
 #define OZ_JOB_B8(BB, T) \
-    split_b_body<BB, true>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.BN, j.padded, j.tiles, bx, by, T)
+    split_b_body<BB, true, false, WIN>(j.X, j.ld, j.rows, j.cols, j.e_in, j.s, j.KC, j.n_kc, j.BN, j.padded, j.tiles, bx, by, T)
 #define OZ_JOB_BN(BB) OZ_JOB_B(BB, false)
 #define OZ_JOB_BT(BB) OZ_JOB_B(BB, true)
 #define OZ_JOB_B8N(BB) OZ_JOB_B8(BB, false)
 #define OZ_JOB_B8T(BB) OZ_JOB_B8(BB, true)
-            if (j.f8) {
+            if (WIN != 1 && j.f8) {
                 if (tr) {
                     OZ_SPLIT_DISPATCH_F8(j.b, OZ_JOB_B8T)
                 } else {
@@ -1018,13 +1019,16 @@ __global__ void __launch_bounds__(kStageThreads, 3)
     }
 }
 
-// Two jobs of one problem (A and B) in one launch: blocks [0, n0) run j0.
-__global__ void __launch_bounds__(kStageThreads) k_stage_pair(const __grid_constant__ StageJob j0,
-                                                              const __grid_constant__ StageJob j1, int n0) {
+// Two jobs of one problem and stage (A and B) in one launch: blocks [0, n0) run j0.  A
+// kernel for each stage and, of stage (b), for splits of one window and the others, three
+// blocks per SM each (one kernel of all bodies took 88 registers and two blocks).
+template <int STAGE, int WIN>
+__global__ void __launch_bounds__(kStageThreads, 3)
+    k_stage_pair(const __grid_constant__ StageJob j0, const __grid_constant__ StageJob j1, int n0) {
     grid_launch_dependents();
     const int bid = blockIdx.x;
-    if (bid < n0) run_stage_job<true, 3>(j0, bid);
-    else run_stage_job<true, 3>(j1, bid - n0);
+    if (bid < n0) run_stage_job<true, STAGE, WIN>(j0, bid);
+    else run_stage_job<true, STAGE, WIN>(j1, bid - n0);
 }
 
 // Pseudo-random doubles in [-1, 1) (splitmix64 of the index): inputs for the
@@ -1088,8 +1092,14 @@ void launch_stage_pair(StageJob j0, StageJob j1, void *stream) {
     stage_grid(j0, &j0.gx, &j0.gy);
     stage_grid(j1, &j1.gx, &j1.gy);
     const int n0 = j0.gx * j0.gy, n1 = j1.gx * j1.gy;
-    if (n0 + n1 > 0)
-        k_stage_pair<<<n0 + n1, kStageThreads, 0, static_cast<cudaStream_t>(stream)>>>(j0, j1, n0);
+    if (n0 + n1 <= 0) return;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (j0.kind != JOB_SPLIT_A && j0.kind != JOB_SPLIT_B)
+        k_stage_pair<1, 0><<<n0 + n1, kStageThreads, 0, st>>>(j0, j1, n0);
+    else if (!j0.f8 && !split_two_windows(j0.b, j0.s))
+        k_stage_pair<2, 1><<<n0 + n1, kStageThreads, 0, st>>>(j0, j1, n0);
+    else
+        k_stage_pair<2, 2><<<n0 + n1, kStageThreads, 0, st>>>(j0, j1, n0);
 }
 
 template <int STAGE>

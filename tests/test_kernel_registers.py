@@ -16,3 +16,9 @@ def _blocks(ozlib, name):
 
 def test_one_launch_split_with_norms_keeps_two_blocks_per_sm(ozlib):
     assert min(_blocks(ozlib, "k_exp_splitILi7ELb0ELb1E")) >= 2
+
+
+def test_stage_pairs_keep_three_blocks_per_sm(ozlib):
+    """Exponents or statistics of two operands, and their splits of one window and of two."""
+    blocks = _blocks(ozlib, "k_stage_pairI")
+    assert len(blocks) == 3 and min(blocks) >= 3
