@@ -26,9 +26,15 @@
 //     hold a pair.  On GB300 a M=128, K=16 UMMA of N columns takes
 //     max(N/2, 32 + N/4) cycles (the tensor pipe, or its operands from shared
 //     memory at 128 bytes a cycle).
-//   * Each block belongs to one issuing warp, so its UMMAs run in order and the
+//   * Each block belongs to one issuing warp, which issues its UMMAs in order, and the
 //     first one after a drain overwrites the accumulator.  Issuers do not wait for
-//     one another beyond the stage ring.
+//     one another beyond the stage ring.  (Assumed: the tensor pipe executes the UMMAs of
+//     one thread on overlapping accumulator columns in the order of issue, also where N and
+//     the first column change.  The PTX text promises that order for equal accumulator and
+//     shape; for the rest it rests on the bit-exact tests against the oracle, in which a
+//     UMMA that overtook the overwriting one would lose its products.)  e4m3 plans of two
+//     blocks deal their UMMAs over all three issuers where one would have most of them
+//     (oz_plan.cpp); those only accumulate, in any order.
 //   * Each block is a drain group with its own period: its tightest bin's, or longer
 //     where the norms of the tile's slices allow it (DrainSchedule).  A block
 //     whose accumulator is being read out holds up its own issuer only; a
@@ -399,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         }
         for (int i = 0; i < g.G; ++i) {
             for (int b = 0; b < 2; ++b) {
-                mbar_init(&gfull[2 * i + b], 1);
+                mbar_init(&gfull[2 * i + b], g.blk_commits[i]);
                 mbar_init(&gempty[2 * i + b], kEpiWarps);
             }
         }
@@ -511,10 +517,10 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
       } else {
         // ---------------------------------------------------- MMA issuers
         // Up to three issuing warps (on different SM sub-partitions).  Each owns some of
-        // the bin blocks and issues all of their UMMAs, so a block's UMMAs run in order:
-        // the first after a drain overwrites the accumulator, and a block that waits for
-        // its drain holds up its own issuer alone, while the others go on to the chunks
-        // that the stage ring holds.  What the warp executes per UMMA decides its rate
+        // the bin blocks and issues all of their UMMAs in order (blocks of zero_mask may be
+        // shared, GemmArgs::blk_commits): the first after a drain overwrites the accumulator,
+        // and a block that waits for its drain holds up its issuer alone, while the others go
+        // on to the chunks that the stage ring holds.  What the warp executes per UMMA decides its rate
         // (it shares its scheduler with four drain warps): four entries at a time, so
         // that their loads and descriptor arithmetic overlap, run warp-wide with one
         // elected lane issuing (55 cycles a UMMA with nothing else on the SM, 77 in a

@@ -122,9 +122,11 @@ struct GemmArgs {
     const float *na, *nb;
     // UMMAs of a K step (pack_op): issuer i's are ops[op_end[i - 1], op_end[i]), those
     // of a block together, first one that spans the block.  Blocks of zero_mask have no
-    // such UMMA (more bins than slices): theirs all accumulate, and the drain warps
-    // store zeros over what they read.
+    // such UMMA (more bins than slices) or UMMAs of several issuers: theirs all accumulate,
+    // and the drain warps store zeros over what they read.  blk_commits: issuers with UMMAs
+    // of the block, each of which commits its own before a drain.
     int op_end[kMaxIssuers];
+    int blk_commits[kMaxGroups];
     // Slices that leave room for one stage (e4m3, s > 20 or so): A comes in `parts` parts
     // of part_slices slices, part_bytes each, through a ring of `stages` parts, B through
     // a ring of kPartStagesB blocks, so that the copies of one chunk overlap the UMMAs of
@@ -165,7 +167,7 @@ struct GemmArgs {
     // below 2^63.  OUT_PAIRS: groups {0, pair_g0}, each modulo 2^64.
     int n_acc;
     int acc_t0[kMaxAcc];
-    int n_iss;  // MMA-issuing warps (1 to 3), each with its own bin blocks
+    int n_iss;  // MMA-issuing warps (1 to 3)
     int pdl;  // launched as a programmatic dependent of the kernel before it in the stream
     double alpha, beta;  // C = alpha * (A B) + beta * C for OUT_RN / OUT_RZ_REF (1, 0: plain store)
 };

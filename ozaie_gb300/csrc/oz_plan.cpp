@@ -406,9 +406,18 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     // the issuing warps, dealt by cost: one thread issues a UMMA about every 60-80
     // cycles at best, more with the drain warps on its scheduler.
     // With A in parts (of sp slices) the UMMAs of each part come together.
+    int heaviest_block = 0;  // UMMAs per K step of the block with the most (after a first call)
     auto build_lists = [&](int sp) {
         p.n_iss = hint.issuers >= 1 && hint.issuers <= kMaxIssuers ? hint.issuers : kMaxIssuers;
-        p.n_iss = std::min(p.n_iss, p.G);
+        // e4m3 plans of two blocks leave the third warp idle and the heavier block's UMMAs to
+        // one warp.  Where those are many (13 a chunk, 0.64 of all, or more) the UMMAs are
+        // dealt one by one over three warps instead, all of them accumulating, so that
+        // their order does not matter.  GEMM at 1500^3, two warps against three: b = 4, s = 18
+        // 494 / 424 us, s = 10 158 / 137, s = 13 242 / 230; below the line s = 11 200 / 221 (11
+        // a chunk), s = 9 with the full pair set 221 / 242 (0.56).
+        const bool shared = p.f8 && p.G == 2 && p.n_iss == kMaxIssuers && sp == s &&
+                            heaviest_block * (p.KC / kpu) >= 13 && 25 * heaviest_block >= 16 * p.mma_per_kstep;
+        if (!shared) p.n_iss = std::min(p.n_iss, p.G);
         p.part_slices = sp;
         p.parts = (s + sp - 1) / sp;
         std::vector<uint32_t> ops[kMaxGroups][kMaxParts];
@@ -416,6 +425,7 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
         int order[kMaxGroups], owner[kMaxGroups];
         p.mma_per_kstep = 0;
         p.zero_mask = 0;
+        auto umma_cost = [&](int nb) { return std::max(0.5 * nb * p.BN, 32.0 + 0.25 * nb * p.BN); };
         for (int g = 0; g < p.G; ++g) {
             const int lo = p.blk_lo[g], hi = lo + p.blk_nb[g] - 1;
             order[g] = g;
@@ -425,21 +435,48 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
                 if (a > e) continue;
                 ops[g][pa / sp].push_back(pack_op(pa, a, e - a + 1, g, 0, false, false));
                 if (first < 0) first = pa / sp;
-                cost[g] += std::max(0.5 * (e - a + 1) * p.BN, 32.0 + 0.25 * (e - a + 1) * p.BN);
+                cost[g] += umma_cost(e - a + 1);
                 ++p.mma_per_kstep;
             }
             auto &f = ops[g][first];
             const auto full =
                 std::find_if(f.begin(), f.end(), [&](uint32_t op) { return op_nb(op) == p.blk_nb[g]; });
-            if (full != f.end()) std::swap(*full, f.front());
+            if (full != f.end() && !shared) std::swap(*full, f.front());
             else p.zero_mask |= 1u << g;
+            p.blk_commits[g] = 1;
+            size_t n = 0;
+            for (const auto &l : ops[g]) n += l.size();
+            heaviest_block = std::max(heaviest_block, static_cast<int>(n));
+        }
+        if (p.mma_per_kstep > kMaxOps) return false;
+        if (shared) {
+            // widest first, each to the least loaded warp; a warp's list is block by block
+            std::vector<uint32_t> all, mine[kMaxIssuers][kMaxGroups];
+            for (int g = 0; g < p.G; ++g) all.insert(all.end(), ops[g][0].begin(), ops[g][0].end());
+            std::stable_sort(all.begin(), all.end(), [](uint32_t x, uint32_t y) { return op_nb(x) > op_nb(y); });
+            for (uint32_t op : all) {
+                const int i = static_cast<int>(std::min_element(load, load + p.n_iss) - load);
+                load[i] += umma_cost(op_nb(op));
+                mine[i][op_blk(op)].push_back(op);
+            }
+            for (int g = 0; g < p.G; ++g) p.blk_commits[g] = 0;
+            for (int i = 0, n = 0; i < p.n_iss; ++i) {
+                for (int g = 0; g < p.G; ++g) {
+                    const auto &l = mine[i][g];
+                    for (size_t k = 0; k < l.size(); ++k)
+                        p.ops[n++] = pack_op(op_p(l[k]), op_lo(l[k]), op_nb(l[k]), g, static_cast<int>(l.size() - k),
+                                             true, true);
+                    if (!l.empty()) ++p.blk_commits[g];
+                }
+                p.op_end[i] = p.part_end[i * kMaxParts] = n;
+            }
+            return true;
         }
         std::stable_sort(order, order + p.G, [&](int x, int y) { return cost[x] > cost[y]; });
         for (int i = 0; i < p.G; ++i) {
             owner[order[i]] = static_cast<int>(std::min_element(load, load + p.n_iss) - load);
             load[owner[order[i]]] += cost[order[i]];
         }
-        if (p.mma_per_kstep > kMaxOps) return false;
         for (int i = 0, n = 0; i < p.n_iss; ++i) {
             for (int j = 0; j < p.parts; ++j) {
                 for (int g = 0; g < p.G; ++g) {
@@ -497,6 +534,7 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
         p.KC = kmin;
         p.stages = 1;
     }
+    build_lists(s);  // again: who issues what depends on the K chunk
     p.fn = nullptr;
     const int vkc = p.f8 ? p.KC / 2 : p.KC;  // the kernel's bf16-equivalent chunk
     for (const Variant &v : kVariants)
@@ -595,6 +633,7 @@ void gemm_args_from_plan(GemmArgs *g, const Plan &p, int out_mode, int *err, uns
         g->blk_lo[i] = p.blk_lo[i];
         g->blk_nb[i] = p.blk_nb[i];
         g->blk_period[i] = p.blk_period[i];
+        g->blk_commits[i] = p.blk_commits[i];
         g->blk_col1[i] = p.blk_col1[i];
     }
     g->dbl_mask = p.dbl_mask;

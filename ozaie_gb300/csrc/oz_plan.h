@@ -35,6 +35,7 @@ struct Plan {
     int blk_period[kMaxGroups] = {0};
     bool norms = false;  // the split takes the slices' norms, and the drains follow them (GemmArgs::na)
     int op_end[kMaxIssuers] = {0};  // the issuers' UMMA lists (GemmArgs)
+    int blk_commits[kMaxGroups] = {0};  // issuers with UMMAs of each block
     int parts = 1, part_slices = 0, part_end[kMaxIssuers * kMaxParts] = {0};  // A in parts (GemmArgs)
     uint32_t part_bytes = 0;
     uint32_t zero_mask = 0;

@@ -404,3 +404,11 @@ def test_data_drains_rule(ozlib):
     assert ozlib.plan_data_drains(128, 304 * c["tile_n"], k + 1, 7, 8, 8) is False
     assert ozlib.plan_data_drains(4096, 4096, 4096, 6, 9, 9) is False
     assert ozlib.plan_data_drains(0, 1, 1, 7, 8, 8) is None
+
+
+@pytest.mark.parametrize("b,s,J", [(4, 18, 18), (4, 9, 9), (3, 18, 19), (2, 10, 11), (1, 16, 17), (4, 7, 7)])
+def test_two_block_e4m3_plans_use_every_issuer(ozlib, b, s, J):
+    """Two blocks owned by a warp each would leave the third issuing warp idle."""
+    c = ozlib.plan_query(1500, 1500, 1500, b, s, J)
+    assert (c["slice_format"], c["blocks"], c["issuers"]) == (1, 2, 3)
+    assert sum(c["block_nb"]) == J

@@ -176,3 +176,18 @@ def test_captured_call_replays(ozlib, M, N, K, mode):
         assert h.sync() == 0, h.last_error()
         assert torch.equal(got, dC)
     h.close()
+
+
+@pytest.mark.parametrize("b,s,J,K", [(4, 18, 18, 9100), (4, 9, 9, 17000), (4, 13, 17, 9100), (4, 7, 7, 70), (2, 10, 11, 1500),
+                                     (3, 18, 19, 1500)])
+@pytest.mark.parametrize("kind", ["random", "largest"])
+def test_two_blocks_dealt_to_three_issuers(ozlib, oracle, b, s, J, K, kind):
+    """e4m3 plans of two bin blocks deal the UMMAs of both over the three issuing warps, all
+    of them accumulating: several drains of each block in a tile, digits of 2^b - 1."""
+    M, N = 133, 70
+    A, B = oracle.gen_phi((M, K), 85, 1.0), oracle.gen_phi((K, N), 86, 1.0)
+    if kind == "largest":
+        A[:], B[:] = np.nextafter(1.0, 0.0), np.nextafter(1.0, 0.0)
+    got, cfg = _run(ozlib, A, B, s, J, bits=b)
+    assert (cfg["slice_format"], cfg["blocks"], cfg["issuers"]) == (1, 2, 3), cfg
+    _same(got, oracle.dgemm(A, B, b, s, J, 0), cfg)
