@@ -717,6 +717,26 @@ def run_reference(args):
     return 0
 
 
+# the record of every workload and comparison; the printed line holds what identifies and
+# checks the headline (a line of all of it is 15 KB, more than a log's tail keeps)
+DETAILS = os.path.join(ROOT, "bench_details.json")
+
+
+def contract_line(rec):
+    """The one line printed on stdout, from the whole record."""
+    keep = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "valid", "stage_ms", "e2e", "gpu_launches", "clocks",
+            "cpu_baseline")
+    line = {k: rec[k] for k in keep if k in rec}
+    acc = rec["accuracy"]
+    line["accuracy"] = {k: v["normwise_rel"] for k, v in acc.items() if v}
+    line["elementwise_mode"] = {"value": rec["elementwise_mode"]["value"], "slices": rec["elementwise_mode"]["slices"]}
+    line["cublas_dgemm"] = rec["cublas_dgemm"]["value"]
+    line["roofline"] = {k: v for k, v in rec["roofline"].items() if k in ("bound", "achieved", "peak", "unit", "frac")}
+    line["details"] = os.path.basename(DETAILS)
+    return line
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -990,7 +1010,9 @@ def main():
         if not args.no_cpu_baseline:
             line["cpu_baseline"] = cpu_baseline(A, B, cfg["slices"], cfg["bins"])
             line["cpu_blas_dgemm"] = cpu_blas_dgemm(A, B)
-        print(json.dumps(line))
+        with open(DETAILS, "w") as f:
+            json.dump(line, f, indent=1)
+        print(json.dumps(contract_line(line)))
     h.close()
     if ws > 1:
         dist.destroy_process_group()
