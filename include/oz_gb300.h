@@ -80,7 +80,8 @@ typedef struct {
     int umma_per_kstep; /* UMMAs per 16-deep K step */
     int block_lo[8]; /* first bin of each block */
     int block_nb[8]; /* bins in each block */
-    int issuers;     /* warps issuing the UMMAs (1 to 3, each those of its own bin blocks) */
+    int issuers;     /* warps issuing the UMMAs (1 to 3, each those of its own bin blocks; e4m3
+                      * plans of two blocks may deal theirs over three) */
     int slice_format;/* 0: bf16 slices (kind::f16); 1: e4m3 slices (kind::f8f6f4, b <= 4) */
     int dbl_blocks;  /* bit g: block g has two accumulator ranges, its UMMAs go on while one drains */
 } ozgb_config;
@@ -269,6 +270,10 @@ int ozgb_plan_query(int M, int N, int K, int bits, int slices, int bins, ozgb_co
 /* Host-only planning query: 1 if a single such product drains by its own digits (its
  * split also takes the slices' norms), 0 if by the worst case, -1 if it has no plan. */
 int ozgb_plan_data_drains(int M, int N, int K, int bits, int slices, int bins);
+/* Test hook: the norms that the last such product drained by (per tile of A, then of B,
+ * and slice: the largest sum of squared digits over a row's or column's K chunk, or a bound
+ * of it), after ozgb_sync.  Returns their number, 0 if it took none; writes at most n. */
+int ozgb_last_norms(ozgb_handle h, float *out, int n);
 /* Host-only precision knob (no device needed): the smallest slice count in
  * [2, 16] whose a-priori normwise error estimate is <= bound (16 if none), from
  * the stage-(a) statistics: row max exponent fields er and row sums of squares

@@ -100,6 +100,7 @@ SIGNATURES = [
     ("ozgb_convert_paired_i64_to_double", _i, [_p, _p, _i, _i, _i, _i, _i]),
     ("ozgb_plan_query", _i, [_i, _i, _i, _i, _i, _i, ctypes.POINTER(OzgbConfig)]),
     ("ozgb_plan_data_drains", _i, [_i, _i, _i, _i, _i, _i]),
+    ("ozgb_last_norms", _i, [_h, _p, _i]),
     ("ozgb_choose_slices", _i, [_p, _p, _i, _p, _p, _i, _p, _p, _i, _i, _dbl, ctypes.POINTER(_dbl)]),
     ("ozgb_choose_slices_ex", _i, [_p, _p, _i, _p, _p, _i, _p, _p, _i, _i, _dbl, _i, _dbl, ctypes.POINTER(_dbl)]),
     ("ozgb_dgemm_device_noalloc", _i, [_i, _i, _i, _p, ctypes.c_long, _p, ctypes.c_long, _p, ctypes.c_long, _i, _p]),

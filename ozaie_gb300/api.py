@@ -190,6 +190,12 @@ class Handle:
         self._check(self._L.ozgb_autotune(self._h, M, N, K, bits, slices, bins, max_candidates, ctypes.byref(c)))
         return c.as_dict()
 
+    def last_norms(self, n):
+        """Test hook: the first n slice norms of the last product that took them (float32)."""
+        out = np.zeros(n, np.float32)
+        have = self._L.ozgb_last_norms(self._h, _ptr(out), int(n))
+        return out if have >= n else None
+
     def launch_count(self):
         n = ctypes.c_longlong()
         self._check(self._L.ozgb_launch_count(self._h, ctypes.byref(n)))

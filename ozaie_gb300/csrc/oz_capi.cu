@@ -1784,6 +1784,16 @@ int ozgb_plan_data_drains(int M, int N, int K, int bits, int slices, int bins) {
     return p ? (p->norms ? 1 : 0) : -1;
 }
 
+int ozgb_last_norms(ozgb_handle h, float *out, int n) {
+    if (!h || !out || n < 0) return 0;
+    std::lock_guard<std::mutex> lk(h->mu);
+    if (!h->have_last || !h->last.norms || !h->norm.p || norm_bytes(h->last) > h->norm.cap) return 0;
+    const int have = static_cast<int>(norm_bytes(h->last) / sizeof(float));
+    cudaSetDevice(h->device);
+    if (cudaMemcpy(out, h->norm.p, sizeof(float) * std::min(n, have), cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
+    return have;
+}
+
 int ozgb_choose_slices(const int32_t *er, const double *ssr, int M, const int32_t *ec, const double *ssc, int N,
                        const double *sa_k, const double *sb_k, int K, int bits, double bound, double *estimate) {
     return ozgb_choose_slices_ex(er, ssr, M, ec, ssc, N, sa_k, sb_k, K, bits, bound, OZGB_CRIT_NORMWISE, 1e-4,

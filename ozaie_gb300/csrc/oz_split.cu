@@ -265,7 +265,9 @@ __device__ __forceinline__ void emit8(const double (&x)[8], int E, bool one_wind
 
 // The largest of the warp's chunk sums of squares per slice into the tile's maxima (bit
 // patterns of non-negative floats order like integers): tiles t0 and, for lanes whose
-// unit lies in the next tile, t0 + 1.
+// unit lies in the next tile, t0 + 1.  (By shuffles: with __reduce_max_sync here nvcc 13.0
+// built a k_split_a, whose maxima pass through a loop, that lost those of two or three
+// slices and left other registers' contents in their place.)
 __device__ __forceinline__ void norm_max(const float *nrm, int s, float *__restrict__ out, int t0, int t) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -275,7 +277,9 @@ __device__ __forceinline__ void norm_max(const float *nrm, int s, float *__restr
 #pragma unroll
         for (int p = 0; p < kMaxNormSlices; ++p)
             if (p < s) {
-                const uint32_t v = __reduce_max_sync(0xffffffffu, t == t0 + d ? __float_as_uint(nrm[p]) : 0u);
+                uint32_t v = t == t0 + d ? __float_as_uint(nrm[p]) : 0u;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
                 if (lane == p) mine = v;
             }
         if (lane < s) {

@@ -86,6 +86,70 @@ def test_data_drains_bit_exact(ozlib, oracle, s, J, kind):
                 assert bad.size == 0, (M, N, K, ta, tb, bad[:4])
 
 
+def _digits(torch, x, s):
+    """Squares of the 7-bit digits of x (units along dimension 0), s x units x K, from the
+    values: x / 2^(E - 1022) has the digits after the point, E a unit's largest exponent."""
+    e = torch.frexp(x.abs().amax(dim=1, keepdim=True))[1]
+    r = torch.ldexp(x.abs(), -e)
+    out = []
+    for _ in range(s):
+        r = r * 128.0
+        d = torch.floor(r)
+        r = r - d
+        out.append((d * d).float())
+    return out
+
+
+@pytest.mark.parametrize("kind", ["random", "largest"])
+@pytest.mark.parametrize("s,J", [(5, 5), (7, 7), (8, 9), (9, 9), (8, 15), (10, 10), (12, 12)])
+def test_norms_are_the_digits_own(ozlib, s, J, kind):
+    """The norms that the drains are planned from, of every tile and slice, against the
+    digits of the operands (s <= 9: all of them in one window): equal, or up to twice where a
+    kernel bounds a chunk by its larger half.  One that is too small would let fp32 sums
+    pass 2^24."""
+    import torch
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(7 * s + J)
+    c = ozlib.plan_query(4096, 4096, 4096, 7, s, J)
+    bn, kc = c["tile_n"], c["k_chunk"]
+    checked = min(s, 7)  # 49 of the 53 bits: no digit depends on how the last is cut
+    for M, N, K, stages in _shapes(s, J, bn):
+        A = torch.rand((M, K), dtype=torch.float64, device=dev, generator=gen) + 2.0 ** -20
+        B = torch.rand((K, N), dtype=torch.float64, device=dev, generator=gen) + 2.0 ** -20
+        if kind == "largest":
+            A.fill_(FULL)
+            B.fill_(FULL)
+        want = []
+        for x, tile in ((A, 128), (B.T, bn)):
+            units, pad = x.shape[0], -x.shape[0] % tile
+            per = []
+            for d in _digits(torch, x, checked):
+                d = torch.nn.functional.pad(d, (0, -K % kc)).reshape(units, -1, kc).sum(dim=2).amax(dim=1)
+                per.append(torch.nn.functional.pad(d, (0, pad)).reshape(-1, tile).amax(dim=1))
+            want.append(torch.stack(per, dim=1))
+        dC = torch.empty((M, N), dtype=torch.float64, device=dev)
+        for ta in (0, 1):
+            for tb in (0, 1):
+                dA, dB = (A.T.contiguous() if ta else A), (B.T.contiguous() if tb else B)
+                h = ozlib.Handle()
+                h.set_slices(s)
+                h.set_bins(J)
+                for _ in range(2):
+                    rc = h.dgemm_ex(ta, tb, M, N, K, 1.0, dA.data_ptr(), dA.shape[1], dB.data_ptr(), dB.shape[1], 0.0,
+                                    dC.data_ptr(), N, torch.cuda.current_stream().cuda_stream)
+                    assert rc == 0, h.last_error()
+                    assert h.sync() == 0, h.last_error()
+                tiles = [w.shape[0] for w in want]
+                got = torch.from_numpy(h.last_norms(s * sum(tiles))).to(dev)
+                h.close()
+                parts = [got[: s * tiles[0]].reshape(-1, s), got[s * tiles[0]:].reshape(-1, s)]
+                for side, (g, w) in enumerate(zip(parts, want)):
+                    g = g[:, :checked]
+                    assert bool((g >= w).all()), (M, N, K, ta, tb, side, (g < w).sum(dim=0).tolist())
+                    top = 2 * w if stages == 1 else w
+                    assert bool((g <= top).all()), (M, N, K, ta, tb, side, (g > top).sum(dim=0).tolist())
+
+
 def test_first_call_after_setup_can_be_captured(ozlib):
     """ozgb_setup reserves every buffer that a call of its shape fills, the slices' norms
     among them: the handle's first call allocates nothing and can be captured."""
