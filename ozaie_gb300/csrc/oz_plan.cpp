@@ -359,8 +359,10 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
         p.model_cycles_per_kstep = part_cost(p.G, p.blk_lo, p.blk_nb);
     }
     // zero B slices that UMMAs spanning whole blocks would read below q = 0 and above
-    // q = s - 1: they are part of the stage size that bounds the slices a product may
-    // have (the UMMA lists below need none)
+    // q = s - 1.  The UMMA lists below need none, but they still count in the stage size
+    // that bounds the slices a product may have and that picks the K chunk and the stages:
+    // the knob ranks schedules by both, so they decide which bits it returns.  (Without
+    // them s = 10 and 11 with J = s would have 32-deep chunks, s = 6 a third stage.)
     int pad_lo = 0, pad_hi = 0;
     for (int g = 0; g < p.G; ++g) {
         const int lo = p.blk_lo[g], hi = lo + p.blk_nb[g] - 1;
@@ -573,7 +575,10 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     // digits' norms, about 15 % more work per value, which pays when a tile drains often
     // by the worst case and the GEMM has more than two tiles per SM.  GEMM at 4096^3, s =
     // 8: p + q <= 8 3.68 -> 3.29 ms, full set 5.67 -> 5.07; calls at 2048^3 490 -> 476 and 830
-    // -> 775 us, but 1024^3 (128 tiles) 89 -> 95, 512 x 512 x 4096 122 -> 127.
+    // -> 775 us, but 1024^3 (128 tiles) 89 -> 95, 512 x 512 x 4096 122 -> 127.  (152: the
+    // GB300's SMs.)  Calls with norms over calls without, s = 3 to 14, K = 400 to 2048: 305 to
+    // 420 tiles 0.96 to 1.13, up to 700 tiles 0.89 to 1.08, above 0.84 to 1.03; the upper ends
+    // are short K and few tiles in one direction.
     p.norms = !p.f8 && b == 7 && s <= kMaxNormSlices && p.n_kc > 2 * p.min_period &&
               static_cast<long long>(p.tiles_m) * p.tiles_n > 2 * 152;
     p.Mp = p.tiles_m * BM;
@@ -653,6 +658,10 @@ bool one_launch_split(const Plan &p, int K) {
     // 483 / 494, 256 x 256 x 512 37.1 / 45.6, but 256 x 256 x 2048 (48 blocks) 55.7 / 51.4,
     // 512 x 512 x 4096 148 / 120 and 3000^3 1384 / 1370; e4m3 slices of b = 3: 64^3 26.9 /
     // 39.9, 2048 x 256 x 1024 279 / 284, 256 x 256 x 2048 141 / 96.
+    // (The blocks are counted for A and B as stored row-major, M x K and K x N: transposes
+    // have Mp / 16 and Np / 8.  The line holds for them too: of 20 shapes from 64 x 64 x 512
+    // to 2048^3 in the four orders, 64 x 64 x 1024 with its 20 blocks among them, none was slower
+    // in one launch than by the separate kernels.)
     const int avoid = 1 + (p.cfg.b == 3 ? 3 : 0);
     const bool two = p.f8 || p.cfg.s * p.cfg.b > 64 - avoid - ((64 - avoid) % p.cfg.b);
     const int blocks = p.Mp / 8 + p.Np / 16;

@@ -170,8 +170,9 @@ struct Schedule {
 };
 
 // Modelled time (ms) of one M x N x K product with a plan on `sms` SMs: the
-// plan's modelled SM cycles per K step (model_cycles_per_kstep, the bin-block cost
-// model fitted to the slice-pair GEMM on GB300) at 2 GHz, over whole waves of
+// plan's modelled SM cycles per K step (model_cycles_per_kstep, a bin-block cost
+// model fitted to an earlier slice-pair GEMM and kept, so that the knob's choices
+// stay) at 2 GHz, over whole waves of
 // tiles, plus the HBM traffic of the split at 6.5 TB/s.
 double plan_time_model(const Plan &p, int M, int N, int K, int sms);
 

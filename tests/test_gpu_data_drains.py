@@ -1,7 +1,8 @@
 """Products whose drains follow the data (the split takes the slices' norms), held bit
-for bit to the oracle on operands that reach the fp32 bound; their buffers, and what the
-autotuner times of them.  They have more than 304 tiles (smaller products, test_gpu_gemm_edges.py's among them, drain by
-the worst case): the shapes here have them in one direction, or in both.
+for bit to the oracle on operands that reach the fp32 bound; the norms themselves; their
+buffers, and what the autotuner times of them.  They have more than 304 tiles (smaller
+products, test_gpu_gemm_edges.py's among them, drain by the worst case): the shapes here
+have them in one direction, or in both.
 """
 import numpy as np
 import pytest

@@ -1,6 +1,6 @@
 """Slice-pair GEMM plans forced through ozgb_set_plan_hint, held bit for bit to
-the oracle: one, two and three issuing warps (the UMMA runs of a K step dealt
-round-robin), bin-block partitions other than the planner's, and double-buffered
+the oracle: one, two and three issuing warps (each issues the UMMAs of its own bin
+blocks), bin-block partitions other than the planner's, and double-buffered
 blocks (a second TMEM accumulator range per block, switched at each drain).
 K = 1100 gives every block several drains per tile; M and N are not multiples of
 the tile."""
