@@ -53,11 +53,11 @@
 //   * Every mbarrier wait is bounded (globaltimer); on expiry the kernel records
 //     an error code, waits for its own copies and MMAs, frees TMEM and returns.
 //
-// At 4096^3 (s = 8, p + q <= 8, 2752 tiles of 128 x 48) the launch takes 3.29 ms (1796
-// TFLOP/s of slice-pair products): 1430 cycles per K step of a tile, of which the UMMAs
-// need 1104.  Without drains it takes 1280; the rest is the issuers and drain warps sharing
-// the schedulers.  (1769 cycles before: UMMAs over whole blocks, 1224 cycles a K step with
-// their zero slices, and drains by the worst case.)
+// At 4096^3 (s = 8, p + q <= 8, 2752 tiles of 128 x 48) the launch takes 3.35 ms (1764
+// TFLOP/s of slice-pair products; 3.27 ms with the autotuner's plan): 1440 cycles per K step
+// of a tile, of which the UMMAs need 1104.  Without drains it takes 1270; the rest is the
+// issuers and drain warps sharing the schedulers.  (1769 cycles before: UMMAs over whole
+// blocks, 1224 cycles a K step with their zero slices, and drains by the worst case.)
 #pragma once
 #include <cuda_runtime.h>
 

@@ -265,7 +265,8 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     // cover, once per drain period.  The model was fitted to an earlier kernel, whose UMMAs
     // spanned whole blocks, and stays as it is: choose_schedule ranks the slice schedules by
     // it, so it decides which bits the knob returns.  Its partitions are still within 2 % of
-    // the best measured (4096^3, s = 8, p + q <= 8: {3,3,3} 3.29 ms, {4,3,2} and {4,5} 3.35).
+    // the best measured (4096^3, s = 8, p + q <= 8: {3,3,3} 3.29 ms, {4,3,2} and {4,5} 3.35,
+    // taken together).
     // The search enumerates the compositions of the bins into G <= 8 blocks whose sizes
     // stay within one of the even split, for every G.
     const int max_groups = kMaxGroups;
@@ -573,8 +574,8 @@ bool make_plan_uncached(int M, int N, int K, const OzConfig &cfg, Plan *out, std
     p.tiles_n = (N + p.BN - 1) / p.BN;
     // Drains that follow the data (single products): the split then also takes the
     // digits' norms, about 15 % more work per value, which pays when a tile drains often
-    // by the worst case and the GEMM has more than two tiles per SM.  GEMM at 4096^3, s =
-    // 8: p + q <= 8 3.68 -> 3.29 ms, full set 5.67 -> 5.07; calls at 2048^3 490 -> 476 and 830
+    // by the worst case and the GEMM has more than two tiles per SM.  GEMM, s = 8: 4096^3
+    // p + q <= 8 3.68 -> 3.35 ms, 4096 x 4096 x 16384 full set 22.5 -> 20.5; calls at 2048^3 490 -> 476 and 830
     // -> 775 us, but 1024^3 (128 tiles) 89 -> 95, 512 x 512 x 4096 122 -> 127.  (152: the
     // GB300's SMs.)  Calls with norms over calls without, s = 3 to 14, K = 400 to 2048: 305 to
     // 420 tiles 0.96 to 1.13, up to 700 tiles 0.89 to 1.08, above 0.84 to 1.03; the upper ends
